@@ -86,11 +86,11 @@ struct es_plan {
   float2 *X = nullptr, *Xnyq = nullptr, *T = nullptr, *Tnyq = nullptr, *tw = nullptr;
   float* dR[2] = {nullptr, nullptr};
   uint32_t* flags = nullptr;
-  uint32_t* centers = nullptr;
+  uint16_t* centres = nullptr;      // sphere mode: bitmap of the previous radius' centres (put_centres)
   float* wtab = nullptr;
   float* partials = nullptr;
-  unsigned* counters = nullptr;     // [0] reductions, [1] centre count, [2] error word
-  float* stats = nullptr;           // [max_radii + 2][4]
+  unsigned* counters = nullptr;     // [0] reductions, [2] error word
+  float* stats = nullptr;           // [max_radii + 2][4]: sum, mean, norm, centres found (unsigned)
   RadDev* rad = nullptr;
   int* thr = nullptr;
   // pinned host staging for per-call parameter uploads
@@ -132,7 +132,7 @@ constexpr int kStatsStride = 4;
 size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
 struct Layout {
-  size_t X, Xnyq, T, Tnyq, T2, Tnyq2, tw, dR0, dR1, flags, centers, wtab, partials, counters, stats, rad, thr, total;
+  size_t X, Xnyq, T, Tnyq, T2, Tnyq2, tw, dR0, dR1, flags, centres, wtab, partials, counters, stats, rad, thr, total;
 };
 
 Layout layout(int n, int max_radii, size_t partial_floats) {
@@ -151,7 +151,7 @@ Layout layout(int n, int max_radii, size_t partial_floats) {
   L.dR0 = take(N * N * N * 4);
   L.dR1 = take(N * N * N * 4);
   L.flags = take(N * N * N / 8);
-  L.centers = take(N * N * N * 4);
+  L.centres = take(N * N * N * 4);
   L.wtab = take((size_t)max_radii * k2n * 4);
   L.partials = take(partial_floats * 4);
   L.counters = take(64);
@@ -245,15 +245,173 @@ __global__ void __launch_bounds__(T) delta_T_kernel(const float2* xH, const floa
   if (es::grid_sum<T>(acc, partials, counter, sred, &total) && threadIdx.x == 0) *ave = total * inv_n3;
 }
 
-// update_sphere_kernel (find_bubbles.cu:73-102): every cell within |d|^2 <= r2max of a centre
-// is ionised.  One warp per centre; lanes split the (dz, dy) rows of the ball.
-__global__ void paint_kernel(const uint32_t* centers, const unsigned* count, uint32_t* flags, int n,
-                             int r2max, int periodic) {
+// update_sphere_kernel (find_bubbles.cu:73-102): every cell within |d|^2 <= r2max of a centre is
+// ionised.  The centres come as a row-aligned bitmap (put_centres), and there are two ways:
+//
+//  * Dilation (many centres): a 32-bit word of the painted row (z, y) is the OR over the ball's
+//    (dz, dy) of the centre row (z + dz, y + dy) widened by w = isqrt(r2max - dz^2 - dy^2) on either
+//    side.  Within the word that is a doubling series of shifts; from outside it only the nearest
+//    centre on each side counts.  Eight lanes share a word, each taking every eighth (dz, dy), and
+//    OR-reduce; words that are full already are left.  The work is N^3 / 32 x pi r^2 short steps
+//    whatever the number of centres.
+//  * One warp per centre (few centres): the warp paints the ball of each centre it finds in its
+//    part of the bitmap, row by row with atomic ORs: work ~ centres x (2 r + 1)^2 / 32 row steps.
+//
+// A step of the first kind costs about a third of one of the second and is shared by 32 cells, so by
+// work alone the lines cross near one centre in 1000 cells; but centres come in clusters, which keep
+// a few warps busy, and at one in 1024 the second way took 62 us at 96^3 (radius 7 cells) where the
+// first takes 22 us.  Below one in 4096 it takes 13 us or less against the first's 28 us.
+// 96^3, 30 radii, z = 8: painting every centre's ball took 196 us a radius (the words of a dense region are
+// ORed ~1000 times), this less than 20 us (10 us at z = 10); the row pass, which used to append the centres to a list through one
+// counter, went from 14.7 to 10.0 us.  Bound by the latency of the loads and of the launch.
+constexpr int kPaintTab = 2048;       // (dz, dy, w) entries of the ball held in shared memory at a time
+constexpr int kPaintSparse = 4096;    // cells per centre from which the warp-per-centre way is taken
+__global__ void __launch_bounds__(256) paint_kernel(const uint32_t* __restrict__ centres, const unsigned* count,
+                                                    uint32_t* flags, int n, int r2max, int periodic) {
+  __shared__ uint32_t tab[kPaintTab];
   const unsigned cnt = *count;
-  if (r2max < 0) return;
-  const long warp = (blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5;
-  const long nwarps = ((long)gridDim.x * blockDim.x) >> 5;
-  for (long ci = warp; ci < (long)cnt; ci += nwarps) es::paint_ball(centers[ci], n, r2max, periodic, flags);
+  if (r2max < 0 || cnt == 0u) return;
+  const int nw = (n + 31) / 32, last_bits = n - 32 * (nw - 1), m = n / 2;
+  const uint32_t last_mask = last_bits == 32 ? 0xffffffffu : (1u << last_bits) - 1u;
+  const uint32_t words = (uint32_t)n * n * nw;          // at most 1024^2 * 32
+  const int lane = threadIdx.x & 31;
+  if ((long)cnt * kPaintSparse < (long)n * n * n) {
+    // words dealt to the warps in turn (four neighbours at a time in large boxes, whose words outnumber
+    // the warps), so that a cluster of centres is shared by many warps
+    const uint32_t nwarps = gridDim.x * (blockDim.x / 32);
+    const uint32_t warp = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
+    const int sh = words > 32u * nwarps ? 2 : 0;
+    for (uint32_t g = warp; (g << sh) < words; g += (32u >> sh) * nwarps) {
+      const uint32_t i = ((g + (uint32_t)(lane >> sh) * nwarps) << sh) + (uint32_t)(lane & ((1 << sh) - 1));
+      uint32_t w = 0u, v0 = 0u;
+      if (i < words) {
+        const uint32_t row = i / (uint32_t)nw, t = i % (uint32_t)nw;
+        w = centres[i] & ((int)t == nw - 1 ? last_mask : 0xffffffffu);
+        v0 = row * (uint32_t)n + 32u * t;
+      }
+      unsigned have = __ballot_sync(0xffffffffu, w != 0u);
+      while (have) {
+        const int src = __ffs(have) - 1;
+        have &= have - 1;
+        const uint32_t vs = __shfl_sync(0xffffffffu, v0, src);
+        for (uint32_t ws = __shfl_sync(0xffffffffu, w, src); ws; ws &= ws - 1)
+          es::paint_ball(vs + (uint32_t)(__ffs(ws) - 1), n, r2max, periodic, flags);
+      }
+    }
+    return;
+  }
+  int rr = es::isqrt_dev(r2max);
+  const int reach = periodic ? n / 2 : n - 1;           // farther offsets only repeat or leave the box
+  if (rr > reach) rr = reach;
+  const int side = 2 * rr + 1, slot = lane & 7;
+  const uint32_t groups = gridDim.x * (blockDim.x / 8);
+  for (int e0 = 0; e0 < side * side; e0 += kPaintTab) {
+    const int ne = min(kPaintTab, side * side - e0);
+    __syncthreads();
+    for (int e = threadIdx.x; e < ne; e += blockDim.x) {
+      const int dz = (e0 + e) / side - rr, dy = (e0 + e) % side - rr;
+      const int rem = r2max - dz * dz - dy * dy;
+      tab[e] = rem < 0 ? 0xffffffffu
+                       : ((uint32_t)(dz + 1023) << 21) | ((uint32_t)(dy + 1023) << 10) | (uint32_t)min(es::isqrt_dev(rem), 1023);
+    }
+    __syncthreads();
+    for (uint32_t g0 = blockIdx.x * (blockDim.x / 8); g0 < words; g0 += groups) {     // uniform over the CTA
+      const uint32_t g = g0 + (threadIdx.x >> 3);
+      const bool mine = g < words;
+      const int t = mine ? (int)(g % (uint32_t)nw) : 0;
+      const int row = mine ? (int)(g / (uint32_t)nw) : 0, cz = row / n, cy = row - cz * n;
+      const int width = t == nw - 1 ? last_bits : 32;
+      const uint32_t mask = t == nw - 1 ? last_mask : 0xffffffffu;
+      // the words to its left and right (-1: the edge of a box that is not periodic)
+      const int ul = t > 0 ? t - 1 : (periodic ? nw - 1 : -1), ur = t < nw - 1 ? t + 1 : (periodic ? 0 : -1);
+      const int wl = ul == nw - 1 ? last_bits : 32, wr = ur == nw - 1 ? last_bits : 32;
+      const uint32_t ml = ul < 0 ? 0u : (ul == nw - 1 ? last_mask : 0xffffffffu);
+      const uint32_t mr = ur < 0 ? 0u : (ur == nw - 1 ? last_mask : 0xffffffffu);
+      // the word's 16 pairs in the pair-major flags: bits o.. of the halves of 64-bit word q (a row
+      // of 24 pairs can run on into word q + 1)
+      const int pr = row * m + 16 * t;
+      const size_t q = (size_t)(pr >> 5);
+      const int o = pr & 31;
+      const bool straddle = o + width / 2 > 32;
+      uint32_t fe = flags[2 * q] >> o, fo = flags[2 * q + 1] >> o;
+      if (straddle) {
+        fe |= flags[2 * q + 2] << (32 - o);
+        fo |= flags[2 * q + 3] << (32 - o);
+      }
+      const uint32_t before = (es::spread16(fe) | (es::spread16(fo) << 1)) & mask;
+      uint32_t acc = mine ? before : mask;
+      for (int eb = 0; eb < ne; eb += 64) {             // 8 entries per lane between the fullness checks
+        if (__all_sync(0xffffffffu, acc == mask)) break;
+        for (int e = eb + slot; e < min(eb + 64, ne) && acc != mask; e += 8) {
+          const uint32_t v = tab[e];
+          if (v == 0xffffffffu) continue;
+          int z = cz + (int)(v >> 21) - 1023, y = cy + (int)((v >> 10) & 2047u) - 1023;
+          const int w = (int)(v & 1023u);
+          if (periodic) {
+            z += z < 0 ? n : (z >= n ? -n : 0);
+            y += y < 0 ? n : (y >= n ? -n : 0);
+          } else if (z < 0 || z >= n || y < 0 || y >= n) {
+            continue;
+          }
+          const uint32_t* src = centres + (size_t)(z * n + y) * nw;
+          const uint32_t x = src[t] & mask;
+          uint32_t xl = src[max(ul, 0)] & ml, xr = src[max(ur, 0)] & mr, res = x;
+          if (x) {
+            if (w >= 31) {
+              res = 0xffffffffu;
+            } else {
+              uint32_t lo = x, hi = x;
+              for (int have = 0; have < w;) {           // shifts 0..have are in
+                const int st = min(have + 1, w - have);
+                lo |= lo << st;
+                hi |= hi >> st;
+                have += st;
+              }
+              res = lo | hi;
+            }
+          }
+          // nearest centre to the left of the word, in the next word unless the ball is wider
+          int base = 0, u = ul, wd = wl;
+          for (int k = 1; !xl && u >= 0 && k < nw && base + wd < w; ++k) {
+            base += wd;
+            u = u > 0 ? u - 1 : (periodic ? nw - 1 : -1);
+            wd = u == nw - 1 ? last_bits : 32;
+            if (u >= 0) xl = src[u] & (u == nw - 1 ? last_mask : 0xffffffffu);
+          }
+          if (xl) {
+            const int nb = w + 1 - (base + wd - (31 - __clz(xl)));
+            if (nb > 0) res |= nb >= 32 ? 0xffffffffu : (1u << nb) - 1u;
+          }
+          // and to the right
+          base = 0; u = ur; wd = wr;
+          for (int k = 1; !xr && u >= 0 && k < nw && base + wd < w; ++k) {
+            base += wd;
+            u = u < nw - 1 ? u + 1 : (periodic ? 0 : -1);
+            wd = u == nw - 1 ? last_bits : 32;
+            if (u >= 0) xr = src[u] & (u == nw - 1 ? last_mask : 0xffffffffu);
+          }
+          if (xr) {
+            const int nb = w + 1 - (base + __ffs(xr));
+            if (nb > 0) res |= nb >= width ? 0xffffffffu : ~((1u << (width - nb)) - 1u);
+          }
+          acc |= res & mask;
+        }
+        // the eight lanes of a word share what they have found
+        acc |= __shfl_xor_sync(0xffffffffu, acc, 1);
+        acc |= __shfl_xor_sync(0xffffffffu, acc, 2);
+        acc |= __shfl_xor_sync(0xffffffffu, acc, 4);
+      }
+      if (mine && slot == 0 && acc != before) {
+        const uint32_t e16 = es::unspread16(acc), o16 = es::unspread16(acc >> 1);
+        atomicOr(flags + 2 * q, e16 << o);
+        atomicOr(flags + 2 * q + 1, o16 << o);
+        if (straddle) {
+          atomicOr(flags + 2 * q + 2, e16 >> (32 - o));
+          atomicOr(flags + 2 * q + 3, o16 >> (32 - o));
+        }
+      }
+    }
+  }
 }
 
 __global__ void erfc_selftest_kernel(const float* x, float* fast, float* lib, int n) {
@@ -512,7 +670,7 @@ int es_plan_create(int n, double box_len, int max_radii, es_plan** out) {
   p->tw = (float2*)(b + L.tw);
   p->dR[0] = (float*)(b + L.dR0); p->dR[1] = (float*)(b + L.dR1);
   p->flags = (uint32_t*)(b + L.flags);
-  p->centers = (uint32_t*)(b + L.centers);
+  p->centres = (uint16_t*)(b + L.centres);
   p->wtab = (float*)(b + L.wtab);
   p->partials = (float*)(b + L.partials);
   p->counters = (unsigned*)(b + L.counters);
@@ -636,6 +794,7 @@ int es_ionize(es_plan* p, const es_ionize_params* prm, float* out, float* nf, vo
   // synchronous row pass and sphere painting
   const int marker = (p->col_variant == 1 && prm->update == 0) ? 1 : 0;
   if (!marker) ES_CUDA(cudaMemsetAsync(p->flags, 0, N3 / 8, s));
+  if (prm->update == 1) ES_CUDA(cudaMemsetAsync(p->stats, 0, (size_t)nr * kStatsStride * 4, s));   // centre counts
   const float inv_zeta = (float)(1.0 / (double)prm->zeta);
   // The intermediate spectrum T is written by the z pass, rewritten by the y pass and read by the
   // row pass; when it fits comfortably in L2 it is kept there (evict_last) while the input
@@ -679,7 +838,6 @@ int es_ionize(es_plan* p, const es_ionize_params* prm, float* out, float* nf, vo
   // x C2R with the excursion-set epilogue of radius r (and the sphere painting of radius r - 1)
   auto row_pass = [&](int r) -> int {
     const TBuf& t = tb[ovl ? (r & 1) : 0];
-    if (prm->update == 1 && r > 0) ES_CUDA(cudaMemsetAsync(p->counters + 1, 0, sizeof(unsigned), s));
     es::OpArgs a = base_args(p);
     a.cin = t.main;
     a.rout = reinterpret_cast<float2*>(p->dR[r & 1]);
@@ -694,8 +852,8 @@ int es_ionize(es_plan* p, const es_ionize_params* prm, float* out, float* nf, vo
     a.inv_zeta = inv_zeta;
     a.update = prm->update;
     a.marker = marker;
-    a.centers = p->centers;
-    a.center_count = p->counters + 1;
+    a.centres = p->centres;
+    a.centre_count = reinterpret_cast<unsigned*>(p->stats) + (size_t)r * kStatsStride + 3;
     a.fc_mean = prm->fc_mean_ps;
     a.normalize = prm->normalize_mean;
     a.hint_in = p->l2_hints ? es::ES_HINT_EVICT_FIRST : es::ES_HINT_NORMAL;
@@ -703,8 +861,8 @@ int es_ionize(es_plan* p, const es_ionize_params* prm, float* out, float* nf, vo
     if (int e = run_op(p, es::OP_ROW_C2R_IONIZE, a, g_row, s)) return e;
     if (prm->update == 1 && r > 0) {
       const int ps = prof_begin(p, ES_PROF_PAINT, s);
-      paint_kernel<<<p->sms * 4, 256, 0, s>>>(p->centers, p->counters + 1, p->flags, p->n,
-                                              p->hr[r - 1].r2max, prm->ref_compat ? 0 : 1);
+      paint_kernel<<<p->sms * 8, 256, 0, s>>>(reinterpret_cast<const uint32_t*>(p->centres), a.centre_count, p->flags,
+                                              p->n, p->hr[r - 1].r2max, prm->ref_compat ? 0 : 1);
       prof_end(p, ps, s);
       ES_CUDA(cudaGetLastError());
     }

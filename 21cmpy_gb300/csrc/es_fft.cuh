@@ -209,14 +209,4 @@ __device__ __forceinline__ float2* fft_lines(float2* a, float2* b, const float2*
   return Stages<N, 0, INV, NL, T, LINE_FAST, ES, LS, TWN, RS>::run(a, b, tw);
 }
 
-// bit spread: 16-bit x -> 32-bit word with x's bits at the even positions
-__device__ __forceinline__ uint32_t spread16(uint32_t x) {
-  x &= 0xFFFFu;
-  x = (x | (x << 8)) & 0x00FF00FFu;
-  x = (x | (x << 4)) & 0x0F0F0F0Fu;
-  x = (x | (x << 2)) & 0x33333333u;
-  x = (x | (x << 1)) & 0x55555555u;
-  return x;
-}
-
 }  // namespace es

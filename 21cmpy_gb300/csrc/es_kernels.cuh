@@ -71,8 +71,9 @@ struct OpArgs {
   int update;                     // 0 centre pixel, 1 sphere painting
   int marker;                     // centre pixel: carry the flag in delta_R's lowest mantissa bit
                                   // instead of the bitmap (TMA row pass)
-  uint32_t* centers;              // sphere mode: centres passing at the previous radius
-  unsigned* center_count;
+  uint16_t* centres;              // sphere mode: bitmap of the centres passing at the previous radius
+                                  // (put_centres), and their number
+  unsigned* centre_count;
   // reductions
   float* partials;
   unsigned* counter;
@@ -293,6 +294,32 @@ __device__ __forceinline__ void set_bits(uint32_t* flags, long a, long b) {
   }
 }
 
+
+// bit spread: 16-bit x -> 32-bit word with x's bits at the even positions, and its inverse
+__device__ __forceinline__ uint32_t spread16(uint32_t x) {
+  x &= 0xFFFFu;
+  x = (x | (x << 8)) & 0x00FF00FFu;
+  x = (x | (x << 4)) & 0x0F0F0F0Fu;
+  x = (x | (x << 2)) & 0x33333333u;
+  x = (x | (x << 1)) & 0x55555555u;
+  return x;
+}
+__device__ __forceinline__ uint32_t unspread16(uint32_t x) {
+  x &= 0x55555555u;
+  x = (x | (x >> 1)) & 0x33333333u;
+  x = (x | (x >> 2)) & 0x0F0F0F0Fu;
+  x = (x | (x >> 4)) & 0x00FF00FFu;
+  x = (x | (x >> 8)) & 0x0000FFFFu;
+  return x;
+}
+
+// Sphere mode's centre bitmap: one bit per voxel, x fastest, every row (z, y) starting on a 32-bit
+// word: (N + 31) / 32 words per row.  A row pass stores 16 bits (8 pairs) at a time, plainly, and
+// writes every piece of every row, so the bitmap needs no clearing and no atomics (the bits past N
+// of a row's last word are never written and never read unmasked).
+template <int N> __device__ __forceinline__ void put_centres(uint16_t* bits, size_t row, int pair, uint32_t even, uint32_t odd) {
+  bits[row * (2 * ((N + 31) / 32)) + pair / 8] = (uint16_t)(spread16(even & 0xFFu) | (spread16(odd & 0xFFu) << 1));
+}
 
 // Sphere painting (update_sphere_kernel, find_bubbles.cu:73-102), one warp per centre: every cell
 // within integer |d|^2 <= r2max of voxel v (linear index, x fastest) is set in the pair-major
@@ -671,16 +698,9 @@ __global__ void __launch_bounds__(RowCfg<N>::T) row_c2r(OpArgs a) {
             if (lane == 0 && (bx | by))
               atomicOr(reinterpret_cast<unsigned long long*>(a.flags) + (base + e) / 32,
                        ((unsigned long long)by << 32) | bx);
-          } else if (bx | by) {
-            const unsigned cnt = __popc(bx) + __popc(by);
-            unsigned first = 0;
-            if (lane == 0) first = atomicAdd(a.center_count, cnt);
-            first = __shfl_sync(0xffffffffu, first, 0);
-            const unsigned lt = (1u << lane) - 1u;
-            const unsigned v0 = (unsigned)((base + e) * 2);
-            unsigned pos = first + __popc(bx & lt) + __popc(by & lt);
-            if (px) a.centers[pos++] = v0;
-            if (py) a.centers[pos] = v0 + 1;
+          } else {
+            if ((lane & 7) == 0) put_centres<N>(a.centres, (size_t)tile * RL + e / M, e % M, bx >> lane, by >> lane);
+            if (lane == 0 && (bx | by)) atomicAdd(a.centre_count, (unsigned)(__popc(bx) + __popc(by)));
           }
         }
         a.rout[base + e] = d;

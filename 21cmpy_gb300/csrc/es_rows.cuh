@@ -259,14 +259,13 @@ __global__ void __launch_bounds__(RowTile<N, V>::T, RowOcc<N, V>::MINB) row2_c2r
             if (HP) {
               // then the previous radius' test on its tile, which has had all of the above to land
               wait_prev();
+              if constexpr (UPD == 0) {
 #pragma unroll
-              for (int r = 0; r < RLAST; ++r) {
-                const int p = j + r * NSL;
-                const float2 pp = pv[l * M + p];
-                const bool px = pp.x >= thr_prev, py = pp.y >= thr_prev;
-                const unsigned bx = __ballot_sync(0xffffffffu, px);
-                const unsigned by = __ballot_sync(0xffffffffu, py);
-                if (UPD == 0) {
+                for (int r = 0; r < RLAST; ++r) {
+                  const int p = j + r * NSL;
+                  const float2 pp = pv[l * M + p];
+                  const unsigned bx = __ballot_sync(0xffffffffu, pp.x >= thr_prev);
+                  const unsigned by = __ballot_sync(0xffffffffu, pp.y >= thr_prev);
                   // pair-major bitmap: one 64-bit word per 32 pairs, even voxels in the low half.
                   // The G lanes of a run hold G consecutive pairs starting at a multiple of G, so
                   // the run lies in one word; its first lane ORs the run's bits in (fire and forget)
@@ -278,22 +277,35 @@ __global__ void __launch_bounds__(RowTile<N, V>::T, RowOcc<N, V>::MINB) row2_c2r
                     atomicOr(reinterpret_cast<unsigned long long*>(a.flags) + pr / 32,
                              ((unsigned long long)gy << (32 + off)) | ((unsigned long long)gx << off));
                   }
-                } else if (bx | by) {
-                  const unsigned cnt = __popc(bx) + __popc(by);
-                  unsigned first = 0;
-                  if (lane == 0) first = atomicAdd(a.center_count, cnt);
-                  first = __shfl_sync(0xffffffffu, first, 0);
-                  const unsigned lt = (1u << lane) - 1u;
-                  const unsigned v0 = (unsigned)((row0 + p) * 2);
-                  unsigned pos = first + __popc(bx & lt) + __popc(by & lt);
-                  if (px) a.centers[pos++] = v0;
-                  if (py) a.centers[pos] = v0 + 1;
                 }
+              } else {
+                // sphere mode: the centres' bitmap, 8 consecutive pairs per store.  A run of fewer
+                // than 8 pairs (G = 4) continues in the next output, r + 1.
+                static_assert(G >= 4, "runs of at least four pairs");
+                constexpr int KR = G >= 8 ? 1 : 8 / G, GP = G >= 8 ? 8 : G;
+                constexpr unsigned PMASK = (1u << GP) - 1u;
+                unsigned cnt = 0u;
+#pragma unroll
+                for (int r0 = 0; r0 < RLAST; r0 += KR) {
+                  unsigned ex = 0u, ey = 0u;
+#pragma unroll
+                  for (int k = 0; k < KR; ++k) {
+                    const float2 pp = pv[l * M + j + (r0 + k) * NSL];
+                    const unsigned bx = __ballot_sync(0xffffffffu, pp.x >= thr_prev);
+                    const unsigned by = __ballot_sync(0xffffffffu, pp.y >= thr_prev);
+                    ex |= ((bx >> (lane & ~(GP - 1))) & PMASK) << (k * GP);
+                    ey |= ((by >> (lane & ~(GP - 1))) & PMASK) << (k * GP);
+                    cnt += __popc(bx) + __popc(by);
+                  }
+                  if ((lane & (GP - 1)) == 0)
+                    put_centres<N>(a.centres, (size_t)(blockIdx.x + it * gridDim.x) * RL + l, j + r0 * NSL, ex, ey);
+                }
+                if (lane == 0 && cnt) atomicAdd(a.centre_count, cnt);
               }
             }
           });
         };
-        // update modes: 0 centre pixel with the bitmap, 1 sphere painting (centre list),
+        // update modes: 0 centre pixel with the bitmap, 1 sphere painting (centre bitmap),
         // 2 centre pixel with the flag carried in delta_R
         if (!has_prev) {
           if (a.marker) epilogue(std::false_type{}, std::integral_constant<int, 2>{});
@@ -342,16 +354,11 @@ __global__ void __launch_bounds__(RowTile<N, V>::T, RowOcc<N, V>::MINB) row2_c2r
                 if (lane == 0 && (bx | by))
                   atomicOr(reinterpret_cast<unsigned long long*>(a.flags) + (pair0 + e) / 32,
                            ((unsigned long long)by << 32) | bx);
-              } else if (bx | by) {
-                const unsigned cnt = __popc(bx) + __popc(by);
-                unsigned first = 0;
-                if (lane == 0) first = atomicAdd(a.center_count, cnt);
-                first = __shfl_sync(0xffffffffu, first, 0);
-                const unsigned lt = (1u << lane) - 1u;
-                const unsigned v0 = (unsigned)((pair0 + e) * 2);
-                unsigned pos = first + __popc(bx & lt) + __popc(by & lt);
-                if (px) a.centers[pos++] = v0;
-                if (py) a.centers[pos] = v0 + 1;
+              } else {
+                // sphere mode: the centres' bitmap, 8 pairs (of one row: M is a multiple of 8) per store
+                if ((lane & 7) == 0)
+                  put_centres<N>(a.centres, (size_t)(blockIdx.x + it * gridDim.x) * RL + row, p, bx >> lane, by >> lane);
+                if (lane == 0 && (bx | by)) atomicAdd(a.centre_count, (unsigned)(__popc(bx) + __popc(by)));
               }
             }
             __stcs(a.rout + pair0 + e, d);                 // streamed: read again only next radius
