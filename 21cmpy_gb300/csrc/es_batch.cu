@@ -163,50 +163,6 @@ __device__ bool tile_reduce(float mine, float* partials, unsigned* arrive, int t
 }
 
 // ---------------------------------------------------------------- P(k) (delta_T.py:84-98)
-// Spherical binning of one z-forward tile of g's spectrum: k^3 |G|^2 / (2 pi^2 V), |k| and the mode
-// count (1, or 2 for kx > 0 of the half spectrum) into per-warp bins, warp-aggregated per bin;
-// arithmetic as the per-box plan's binning.
-template <int N, int TI>
-__device__ __forceinline__ void pk_bin_tile(const BoxDev& b, int plane, int c, bool nyq, const float2* Rr, float* bins,
-                                            float* scratch, const int* sthr) {
-  constexpr int M = N / 2;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int NB = b.nbins;
-  float* wb = bins + warp * NB * 3;
-  float* ws = scratch + warp * 32 * 4;
-  const float inv = 1.0f / (2.0f * 9.8696044010893586f * b.volume);
-  for (int e = threadIdx.x; e < N * TI; e += BT) {       // whole warps iterate together
-    const int row = e / TI, col = e % TI;
-    int k2;
-    float wgt;
-    if (!nyq) { const int kx = c * TI + col; k2 = wrap2<N>(row) + wrap2<N>(plane) + kx * kx; wgt = kx == 0 ? 1.f : 2.f; }
-    else { k2 = wrap2<N>(row) + wrap2<N>(c * TI + col) + M * M; wgt = 1.f; }
-    int lo = 0, hi = b.nbins;                            // first bin with k2 <= thr[bin]
-    while (lo < hi) { const int mid = (lo + hi) >> 1; if (k2 <= sthr[mid]) hi = mid; else lo = mid + 1; }
-    int bin = lo;
-    if (k2 == 0) bin = b.nbins;                          // the mean (k = 0) is excluded
-    const float2 gk = Rr[e];
-    const float km = b.dk * sqrtf((float)k2);
-    ws[lane * 4 + 0] = wgt * km * km * km * (gk.x * gk.x + gk.y * gk.y) * inv;
-    ws[lane * 4 + 1] = wgt * km;
-    reinterpret_cast<unsigned*>(ws)[lane * 4 + 2] = (unsigned)wgt;
-    const unsigned peers = __match_any_sync(0xffffffffu, bin);
-    __syncwarp();
-    if (bin < b.nbins && lane == __ffs(peers) - 1) {
-      float p = 0.f, k = 0.f;
-      unsigned n = 0u;
-      unsigned m = peers;
-      while (m) {
-        const int l = __ffs(m) - 1;
-        m &= m - 1;
-        p += ws[l * 4 + 0]; k += ws[l * 4 + 1]; n += reinterpret_cast<const unsigned*>(ws)[l * 4 + 2];
-      }
-      wb[bin] += p; wb[NB + bin] += k; reinterpret_cast<unsigned*>(wb)[2 * NB + bin] += n;
-    }
-    __syncwarp();
-  }
-}
-
 // The tile's bins (warps summed in a fixed order) go to its slot of the per-tile partials; the
 // last tile of the pass to arrive sums the slots in tile order (lanes over tiles, a fixed
 // butterfly), so P(k) does not depend on which CTA ran which tile, and writes the bin means.
@@ -350,7 +306,11 @@ __device__ __noinline__ void b_col_chunk(const BoxDev& b, int radius, int t0, in
     if (tile + 2 < t1) issue(tile + 2, abuf + ((tile - t0 + 2) % 3) * N * TI);   // tile - 1's buffer
     float2* Rr = fft_lines<N, INV, TI, BT, true, TI, 1, N, BCol<N>::RS>(A, B, tw);
     if (PK) {
-      pk_bin_tile<N, TI>(b, g.plane, g.c, g.nyq, Rr, bins, scratch, sthr);
+      const int NB = b.nbins, kx = g.c * TI + threadIdx.x % TI;
+      float* wb = bins + (threadIdx.x >> 5) * 3 * NB;
+      const int ck2 = g.nyq ? wrap2<N>(kx) + M * M : wrap2<N>(g.plane) + kx * kx;
+      pk_bin_columns<N, TI, BT>(Rr, ck2, g.nyq || kx == 0 ? 1u : 2u, sthr, NB, b.dk, b.volume, wb, wb + NB,
+                                reinterpret_cast<unsigned*>(wb) + 2 * NB);
       pk_tile_done<N>(b, tile, bins, scratch);
     } else if (OP == B_COL_Y_FWD && g.c == 0) {
       for (int e = threadIdx.x; e < N * TI; e += BT) {

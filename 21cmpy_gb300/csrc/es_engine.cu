@@ -89,7 +89,7 @@ struct es_plan {
   uint16_t* centres = nullptr;      // sphere mode: bitmap of the previous radius' centres (put_centres)
   float* wtab = nullptr;
   float* partials = nullptr;
-  unsigned* counters = nullptr;     // [0] reductions, [2] error word
+  unsigned* counters = nullptr;     // [0] reductions, [2] error word, [16..63] P(k) groups
   float* stats = nullptr;           // [max_radii + 2][4]: sum, mean, norm, centres found (unsigned)
   RadDev* rad = nullptr;
   int* thr = nullptr;
@@ -154,7 +154,7 @@ Layout layout(int n, int max_radii, size_t partial_floats) {
   L.centres = take(N * N * N * 4);
   L.wtab = take((size_t)max_radii * k2n * 4);
   L.partials = take(partial_floats * 4);
-  L.counters = take(64);
+  L.counters = take(256);
   L.stats = take((size_t)(max_radii + 2) * kStatsStride * 4);
   L.rad = take((size_t)max_radii * sizeof(RadDev));
   L.thr = take(es::PK_MAX_BINS * 4);
@@ -698,7 +698,7 @@ int es_plan_create(int n, double box_len, int max_radii, es_plan** out) {
     tw[m] = make_float2((float)std::cos(ang), (float)std::sin(ang));
   }
   if (cudaMemcpy(p->tw, tw.data(), n * sizeof(float2), cudaMemcpyHostToDevice) != cudaSuccess ||
-      cudaMemset(p->counters, 0, 64) != cudaSuccess || cudaMemset(p->stats, 0, (size_t)(max_radii + 2) * kStatsStride * 4) != cudaSuccess)
+      cudaMemset(p->counters, 0, 256) != cudaSuccess || cudaMemset(p->stats, 0, (size_t)(max_radii + 2) * kStatsStride * 4) != cudaSuccess)
     return cleanup(fail(ES_E_CUDA, "es_plan_create: initial upload failed"));
   if (cudaEventRecord(p->staged, 0) != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess)
     return cleanup(fail(ES_E_CUDA, "es_plan_create: synchronisation failed"));

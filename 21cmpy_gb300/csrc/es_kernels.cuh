@@ -360,12 +360,98 @@ template <int N> __device__ __forceinline__ int wrap2(int k) {
 // third row (a bin of a 512^3 box holds more than 2^24 modes, beyond float32's exact integers).
 __device__ __forceinline__ unsigned* pk_counts(float* bins) { return reinterpret_cast<unsigned*>(bins) + 2 * PK_MAX_BINS; }
 
-// Per-CTA bins (fixed warp order) -> partials -> the last CTA to arrive adds the partials in a
-// fixed order and writes ps_ave, k_ave and the count (rounded to float32 once, at the end).
+// Spherical binning of one z-forward tile (TI columns, N values of kz): k^3 |G|^2 / (2 pi^2 V), |k| and
+// the mode count, summed per bin into the warp's own bins.  kz and N - kz have the same |k|, so a
+// thread takes the pair as one value: NSEG = T / TI threads share a column, each with KS consecutive
+// |kz| (1 .. N/2, and 0 with the first).  |k|^2 rises along them, so the warp walks the bins upward
+// together from the lowest any lane holds, four at a time: each lane adds up its values below each
+// bin's threshold (`thr`, non-decreasing) and one transposing butterfly sums the lanes' eight values
+// in a fixed order (deterministic).  Most tiles hold two or three bins, so a tile costs about
+// N/2 / NSEG short steps and one butterfly; the few tiles at small k hold most bins, and set the tail;
+// merging lanes at every bin change of any of them, the earlier way, cost more than the transform
+// (z forward + binning at 256^3: 99 us with 20 bins and 232 us with 100, the pass without binning 21 us;
+// now 45 us and 62 us).  ck2: the column's ky^2 + kx^2; wgt: modes a value stands for.
+template <int N, int TI, int T>
+__device__ __forceinline__ void pk_bin_columns(const float2* g, int ck2, unsigned wgt, const int* thr, int nbins, float dk,
+                                               float volume, float* sum_p, float* sum_k, unsigned* count) {
+  constexpr int M = N / 2, NSEG = T / TI, KS = (M + NSEG - 1) / NSEG;
+  static_assert(NSEG * TI == T && T % 32 == 0, "threads must cover whole columns");
+  const float inv = 1.0f / (2.0f * 9.8696044010893586f * volume);
+  const int col = threadIdx.x % TI, seg = threadIdx.x / TI;
+  int k = seg == 0 ? 0 : seg * KS + 1;
+  const int end = min(seg * KS + KS, M);                 // last |kz| of this thread
+  if (k == 0 && ck2 == 0) k = 1;                         // the mean (k = 0) is excluded
+  // lowest bin of the thread's first value, then of the warp
+  int lo = 0, hi = nbins;
+  const int first = k * k + ck2;
+  while (lo < hi) { const int mid = (lo + hi) >> 1; if (first <= thr[mid]) hi = mid; else lo = mid + 1; }
+  if (k > end) lo = nbins;
+  const int lane = threadIdx.x & 31, v = lane >> 2;
+  for (int b = __reduce_min_sync(0xffffffffu, lo); b < nbins; b += 4) {
+    float w[8];                                          // sums of bins b .. b + 3, then their |k|
+    unsigned tot[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int top = b + q < nbins ? thr[b + q] : -1;
+      float ap = 0.f, ak = 0.f;
+      unsigned an = 0u;
+      for (; k <= end; ++k) {
+        const int k2 = k * k + ck2;
+        if (k2 > top) break;
+        const float2 u = g[k * TI + col];
+        float pw = u.x * u.x + u.y * u.y;
+        unsigned n = wgt;
+        if (k > 0 && k < M) {
+          const float2 m = g[(N - k) * TI + col];
+          pw += m.x * m.x + m.y * m.y;
+          n += wgt;
+        }
+        const float km = dk * sqrtf((float)k2);
+        ap += (float)wgt * km * km * km * pw * inv;
+        ak += (float)n * km;
+        an += n;
+      }
+      w[q] = ap;
+      w[4 + q] = ak;
+      tot[q] = __reduce_add_sync(0xffffffffu, an);
+    }
+    if (tot[0] | tot[1] | tot[2] | tot[3]) {
+      // transposing butterfly: each step halves the values a lane keeps; lanes 4 v .. 4 v + 3 end
+      // up with value v
+#pragma unroll
+      for (int h = 4, o = 16; h >= 1; h >>= 1, o >>= 1) {
+#pragma unroll
+        for (int q = 0; q < h; ++q) {
+          const float keep = lane & o ? w[q + h] : w[q], give = lane & o ? w[q] : w[q + h];
+          w[q] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+        }
+      }
+      w[0] += __shfl_xor_sync(0xffffffffu, w[0], 2);
+      w[0] += __shfl_xor_sync(0xffffffffu, w[0], 1);
+      const int bin = b + (v & 3);
+      if (bin < nbins) {
+        if ((lane & 3) == 0) (v < 4 ? sum_p : sum_k)[bin] += w[0];
+        if ((lane & 3) == 1 && v < 4) count[bin] += v & 2 ? (v & 1 ? tot[3] : tot[2]) : (v & 1 ? tot[1] : tot[0]);
+      }
+    }
+    if (__all_sync(0xffffffffu, k > end)) break;
+  }
+}
+
+// Per-CTA bins (fixed warp order) -> partials -> the last CTA of each group of consecutive CTAs adds
+// the group's partials -> the last group adds the groups', each in a fixed order, and writes ps_ave,
+// k_ave and the count (rounded to float32 once, at the end).  About sqrt(grid) CTAs form a group, so
+// either step reads ~20 partials per value, all in flight at once: the single last CTA that read all
+// 304 of them one after the other took 45 us of the 256^3 pass with 20 bins and 160 us with 100.
+constexpr int kPkGroups = 48;                         // arrival counters of the groups, from counter[16]
 template <int T>
 __device__ __forceinline__ void pk_finish(float* bins, const OpArgs& a) {
   __syncthreads();
-  const int nb3 = 3 * a.nbins;
+  const int nb3 = 3 * a.nbins, grid = (int)gridDim.x;
+  int gs = 1;
+  while (gs * gs < grid || gs * kPkGroups < grid) ++gs;
+  const int groups = (grid + gs - 1) / gs, grp = (int)blockIdx.x / gs, members = min(gs, grid - grp * gs);
+  float* part2 = a.partials + (size_t)grid * nb3;     // the groups' sums
   for (int idx = threadIdx.x; idx < nb3; idx += T) {
     const int q = idx / a.nbins, bin = idx % a.nbins;
     if (q < 2) {
@@ -379,30 +465,40 @@ __device__ __forceinline__ void pk_finish(float* bins, const OpArgs& a) {
     }
   }
   __shared__ unsigned s_last;
+  // `parts` partials starting at src: value idx, as float or (counts) exact unsigned
+  auto add_up = [&](const float* src, int parts, int idx) {
+    if (idx < 2 * a.nbins) {
+      float s = 0.f;
+#pragma unroll 8
+      for (int c = 0; c < parts; ++c) s += __ldcg(src + (size_t)c * nb3 + idx);
+      return s;
+    }
+    unsigned s = 0u;                                  // at most 1024^3 modes
+#pragma unroll 8
+    for (int c = 0; c < parts; ++c) s += __float_as_uint(__ldcg(src + (size_t)c * nb3 + idx));
+    return __uint_as_float(s);
+  };
   __threadfence();
   __syncthreads();
-  if (threadIdx.x == 0) s_last = (atomicAdd(a.counter, 1u) == gridDim.x - 1) ? 1u : 0u;
+  if (threadIdx.x == 0) s_last = (atomicAdd(a.counter + 16 + grp, 1u) == (unsigned)members - 1) ? 1u : 0u;
   __syncthreads();
   if (!s_last) return;
   __threadfence();
-  // One warp per value: lanes stride over the CTAs' partials (32 loads in flight instead of one
-  // dependent chain per thread), then a fixed butterfly: deterministic
+  for (int idx = threadIdx.x; idx < nb3; idx += T)
+    part2[(size_t)grp * nb3 + idx] = add_up(a.partials + (size_t)grp * gs * nb3, members, idx);
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    a.counter[16 + grp] = 0u;
+    s_last = (atomicAdd(a.counter, 1u) == (unsigned)groups - 1) ? 1u : 0u;
+  }
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
   float* tot = bins;                                  // reuse: [3 * nbins]
-  const int lane = threadIdx.x & 31;
-  for (int idx = threadIdx.x >> 5; idx < nb3; idx += T / 32) {
-    if (idx < 2 * a.nbins) {
-      float s = 0.f;
-      for (int b = lane; b < (int)gridDim.x; b += 32) s += __ldcg(a.partials + (size_t)b * nb3 + idx);
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-      if (lane == 0) tot[idx] = s;
-    } else {
-      unsigned long long s = 0ull;
-      for (int b = lane; b < (int)gridDim.x; b += 32) s += __float_as_uint(__ldcg(a.partials + (size_t)b * nb3 + idx));
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-      if (lane == 0) tot[idx] = __ull2float_rn(s);
-    }
+  for (int idx = threadIdx.x; idx < nb3; idx += T) {
+    const float s = add_up(part2, groups, idx);
+    tot[idx] = idx < 2 * a.nbins ? s : __uint2float_rn(__float_as_uint(s));
   }
   __syncthreads();
   for (int bin = threadIdx.x; bin < a.nbins; bin += T) {

@@ -327,76 +327,11 @@ __global__ void __launch_bounds__(ColTile<N, V>::T, ColTile<N, V>::MINB) col_tma
     (void)RESULT_IN_W;
 
     if (MODE == COL_Z_FWD_PK) {
-      // Each thread runs down KR consecutive kz of one column, where |k| changes slowly, and
-      // accumulates one bin at a time; when a lane's bin changes, the warp merges the finished
-      // runs of all lanes that changed (grouped by bin, summed in lane order: deterministic).
-      constexpr int NSEG = T / TI;                          // k segments per column
-      constexpr int KR = (N + NSEG - 1) / NSEG;             // kz per segment (last may be short)
-      static_assert(NSEG * TI == T, "threads must cover whole columns");
-      const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-      float* wb = bins + warp * PK_MAX_BINS * 3;
-      // the warps' merge scratch [warps][32][4] lives in whichever of S / W the transform left free
-      // (this tile's input buffer is loaded again only after the barrier that ends the tile), so
-      // the P(k) pass needs no shared memory of its own beyond the bins and fits two CTAs per SM
-      float* ws = reinterpret_cast<float*>(out == W ? S : W) + warp * 32 * 4;
-      const float inv = 1.0f / (2.0f * 9.8696044010893586f * a.volume);
-      const int col = threadIdx.x % TI, k0 = (threadIdx.x / TI) * KR;
-      int ck2;
-      float wgt;
-      if (!t.nyq) { const int kx = t.c * TI + col; ck2 = wrap2<N>(t.plane) + kx * kx; wgt = kx == 0 ? 1.f : 2.f; }
-      else { ck2 = wrap2<N>(t.c * TI + col) + M * M; wgt = 1.f; }
-      int cur = -1;
-      int pos = -1;                                          // bin of the previous k in this run
-      float ap = 0.f, ak = 0.f;
-      unsigned an = 0u;                                      // mode count: exact integer
-      const unsigned wgt_u = (unsigned)wgt;
-      auto flush = [&](bool mine) {
-        const int key = mine ? cur : -1;
-        const unsigned peers = __match_any_sync(0xffffffffu, key);
-        ws[lane * 4 + 0] = ap; ws[lane * 4 + 1] = ak; reinterpret_cast<unsigned*>(ws)[lane * 4 + 2] = an;
-        __syncwarp();
-        if (mine && lane == __ffs(peers) - 1) {
-          float p = 0.f, k = 0.f;
-          unsigned n = 0u;
-          unsigned m = peers;
-          while (m) {
-            const int l = __ffs(m) - 1;
-            m &= m - 1;
-            p += ws[l * 4 + 0]; k += ws[l * 4 + 1]; n += reinterpret_cast<const unsigned*>(ws)[l * 4 + 2];
-          }
-          wb[cur] += p; wb[PK_MAX_BINS + cur] += k; pk_counts(wb)[cur] += n;
-        }
-        __syncwarp();
-      };
-      for (int q = 0; q < KR; ++q) {                         // warp-uniform trip count
-        const int k = k0 + q;
-        const bool valid = k < N;
-        const int k2 = wrap2<N>(valid ? k : 0) + ck2;
-        // first bin with k2 <= thr[bin]: a binary search for the run's first k, then a walk from the
-        // previous k's bin (|k|^2 rises, then falls past N/2, so the bin moves by a step or two)
-        int lo = pos;
-        if (lo < 0) {
-          int hi = a.nbins;
-          lo = 0;
-          while (lo < hi) { const int mid = (lo + hi) >> 1; if (k2 <= sthr[mid]) hi = mid; else lo = mid + 1; }
-        } else {
-          while (lo < a.nbins && k2 > sthr[lo]) ++lo;
-          while (lo > 0 && k2 <= sthr[lo - 1]) --lo;
-        }
-        pos = lo;
-        const int bin = (k2 == 0 || !valid) ? a.nbins : lo;    // the mean (k = 0) is excluded
-        const bool change = bin != cur;
-        if (__any_sync(0xffffffffu, change && cur >= 0 && cur < a.nbins))
-          flush(change && cur >= 0 && cur < a.nbins);
-        if (change) { cur = bin; ap = ak = 0.f; an = 0u; }
-        if (!valid) continue;
-        const float2 g = out[k * TI + col];
-        const float km = a.dk * sqrtf((float)k2);
-        ap += wgt * km * km * km * (g.x * g.x + g.y * g.y) * inv;
-        ak += wgt * km;
-        an += wgt_u;
-      }
-      flush(cur >= 0 && cur < a.nbins);
+      float* wb = bins + (threadIdx.x >> 5) * PK_MAX_BINS * 3;
+      const int kx = t.c * TI + threadIdx.x % TI;            // the column's x index (Nyquist plane: its y index)
+      const int ck2 = t.nyq ? wrap2<N>(kx) + M * M : wrap2<N>(t.plane) + kx * kx;
+      pk_bin_columns<N, TI, T>(out, ck2, t.nyq || kx == 0 ? 1u : 2u, sthr, a.nbins, a.dk, a.volume, wb, wb + PK_MAX_BINS,
+                               pk_counts(wb));
       __syncthreads();
     } else {
       if (MODE == COL_Y_FWD && t.c == 0) {
