@@ -2,6 +2,7 @@
 // -DES_N=<N>; each object exports es_launch_<N>(), which es_engine.cu dispatches to.
 #include "es_kernels.cuh"
 #include "es_tma.cuh"
+#include "es_colw.cuh"
 #include "es_rows.cuh"
 #include "es_ops.h"
 
@@ -42,13 +43,18 @@ template <int N, int MODE, int RS>
 static cudaError_t launch_col_tma(const OpArgs& a, cudaStream_t s) {
   if (a.col_tile == 1) return launch<col_tma<N, MODE, 1, RS>>(TmaSmem<N, MODE, 1>::bytes, a, ColTile<N, 1>::T, s);
   if (a.col_tile == 2) return launch<col_tma<N, MODE, 2, RS>>(TmaSmem<N, MODE, 2>::bytes, a, ColTile<N, 2>::T, s);
-  return launch<col_tma<N, MODE, 0, RS>>(TmaSmem<N, MODE, 0>::bytes, a, ColTile<N, 0>::T, s);
+  // tile shape 0 with the large radices is the warp-per-columns form at the sizes that have it
+  if constexpr (ColW<N>::TI > 0 && RS == 0 && MODE != COL_Z_FWD_PK) return cudaErrorInvalidValue;
+  else return launch<col_tma<N, MODE, 0, RS>>(TmaSmem<N, MODE, 0>::bytes, a, ColTile<N, 0>::T, s);
 }
 
 // The per-radius column passes also come with the small-radix schedule (ES_OPT_COL_RADIX).
 template <int N, int MODE>
 static cudaError_t launch_col(const OpArgs& a, cudaStream_t s) {
   if (a.variant == 0) return launch<col_pass<N, MODE>>(ColSmem<N, MODE>::bytes, a, ColCfg<N>::T, s);
+  if constexpr (ColW<N>::TI > 0 && MODE != COL_Z_FWD_PK) {
+    if (a.col_warp) return launch<col_warp<N, MODE>>(ColWSmem<N, MODE>::bytes, a, ColWSmem<N, MODE>::T, s);
+  }
   if constexpr (MODE == COL_Z_INV_FILTER || MODE == COL_Y_INV) {
     if (a.col_radix == 1) return launch_col_tma<N, MODE, 1>(a, s);
   }
@@ -134,6 +140,7 @@ static void geometry(OpGeometry* g) {
   g->col_smem = ColSmem<N, COL_Z_INV_FILTER>::bytes;
   g->col_smem_pk = ColSmem<N, COL_Z_FWD_PK>::bytes;
   g->row_smem = RowSmem<N>::bytes;
+  g->colw_ti = ColW<N>::TI;
   col_geometry<N, 0>(g);
   col_geometry<N, 1>(g);
   col_geometry<N, 2>(g);

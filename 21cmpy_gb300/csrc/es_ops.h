@@ -29,6 +29,7 @@ struct OpGeometry {
   // TMA column passes, per tile variant (ES_OPT_COL_TILE)
   int tcol_ti[kColTileVariants], tcol_threads[kColTileVariants], tcol_tiles_z[kColTileVariants];
   int tcol_tiles_y[kColTileVariants], tcol_smem[kColTileVariants], tcol_smem_pk[kColTileVariants];
+  int colw_ti;                      // tile width of the warp-per-columns passes (es_colw.cuh), 0: none at this size
   // TMA row passes, per tile variant (ES_OPT_ROW_TILE)
   int trow_tiles[kRowTileVariants], trow_threads[kRowTileVariants], trow_smem[kRowTileVariants];
   int trow_smem_prev[kRowTileVariants];
