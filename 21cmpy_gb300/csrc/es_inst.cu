@@ -4,6 +4,7 @@
 #include "es_tma.cuh"
 #include "es_colw.cuh"
 #include "es_rows.cuh"
+#include "es_roww.cuh"
 #include "es_ops.h"
 
 #ifndef ES_N
@@ -79,7 +80,12 @@ static cudaError_t launch_c2r_tma(const OpArgs& a, cudaStream_t s) {
     case 1: return launch<row2_c2r<N, EPI, 1, RS>>(Row2Smem<N, P, 1>::bytes, a, RowTile<N, 1>::T, s);
     case 2: return launch<row2_c2r<N, EPI, 2, RS>>(Row2Smem<N, P, 2>::bytes, a, RowTile<N, 2>::T, s);
     case 3: return launch<row2_c2r<N, EPI, 3, RS>>(Row2Smem<N, P, 3>::bytes, a, RowTile<N, 3>::T, s);
-    default: return launch<row2_c2r<N, EPI, 0, RS>>(Row2Smem<N, P, 0>::bytes, a, RowTile<N, 0>::T, s);
+    default:
+      // tile shape 0 with the large radices is the warp-per-rows form at the sizes that have it
+      if constexpr (RowW<N>::NP > 0 && RS == 0)
+        return launch<row_warp_c2r<N, EPI>>(RowWCfg<N>::bytes, a, RowWCfg<N>::T, s);
+      else
+        return launch<row2_c2r<N, EPI, 0, RS>>(Row2Smem<N, P, 0>::bytes, a, RowTile<N, 0>::T, s);
   }
 }
 

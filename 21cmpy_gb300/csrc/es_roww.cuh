@@ -1,0 +1,302 @@
+// Row C2R pass with one warp per few rows (sm_103a): half-spectrum rows -> real rows, with the
+// excursion-set epilogue or a plain store.  A warp owns RW = 32 / NSL rows of every tile of its CTA (NSL:
+// butterflies of the last stage), copies them in by itself (1-D bulk copies on its own mbarriers, the
+// next tile's rows and previous-radius delta_R in flight), and takes them through the Hermitian split,
+// both Stockham stages and the epilogue with warp-level synchronisation only:
+//
+//   * the split feeds the first stage in registers: a lane reads the elements of its butterfly and
+//     their mirror images and forms Z[e] = (X[e] + conj X[M-e]) + U[e] (X[e] - conj X[M-e]) itself;
+//   * the one exchange between the stages goes through the rows' own buffer, skewed so that neither
+//     side has bank conflicts;
+//   * the second stage's outputs stay in registers for the erfc sum, the previous radius' test and
+//     the store.
+//
+// What bounds it: instruction issue (the erfc sum is half of it).  The older form (es_rows.cuh) spent
+// 1018 warp instructions per tile and warp at 256^3, with four CTA barriers a tile (issue active 60 %).
+// Thread for thread, the last stage, the running sums and the grid are the older form's, so the
+// grid-wide sums come out the same bit for bit.
+#pragma once
+#include "es_rows.cuh"
+
+namespace es {
+
+// NP: previous-radius buffers per warp; 0: the size keeps the older form (two stages with whole
+// warps of butterflies are needed; the small sizes are a single short tile per CTA).
+template <int N> struct RowW { static constexpr int NP = 0; };
+template <> struct RowW<128> { static constexpr int NP = 1; };   // one tile per CTA, mostly
+template <> struct RowW<256> { static constexpr int NP = 2; };
+template <> struct RowW<512> { static constexpr int NP = 2; };
+
+template <int N> struct RowWCfg {
+  static constexpr int M = N / 2, RL = Row2Cfg<N>::RL, NP = RowW<N>::NP;
+  static constexpr int R0 = Plan<M, 0>::radix[0], R1 = Plan<M, 0>::radix[Plan<M, 0>::stages - 1];
+  static constexpr int NSL = R0;                         // butterflies per row of the last of two stages
+  static constexpr int RW = 32 / NSL;                    // rows per warp
+  static constexpr int NW = RL / RW, T = 32 * NW;        // warps and threads of a CTA
+  static constexpr bool HALF = RW * R1 * 2 == 32;        // first stage: two lanes per butterfly
+  // rows of 64 elements: every other row starts half a bank cycle later, so 16 lanes on two rows
+  // touch all 32 banks
+  static constexpr int PITCH = M + (NSL == 8 ? 8 : 0);   // complex elements
+  static constexpr int XBUF = RW * PITCH * 8;            // bytes of one buffer
+  static constexpr int TW = (R1 - 1) * NSL;              // last stage's twiddles
+  // [U | twiddles | per warp: 4 mbarriers | per warp: 2 spectrum, NP previous-radius buffers]
+  static constexpr int BARS = (M + TW) * 8, BUFS = (BARS + NW * 32 + 127) / 128 * 128;
+  static constexpr int bytes = BUFS + NW * (2 + NP) * XBUF + 128;
+};
+
+// Grid-wide sum with the summation order of a CTA of TV threads whose warps past NW hold zeros
+// (grid_sum<TV>, es_kernels.cuh).
+template <int TV, int NW>
+__device__ __forceinline__ bool grid_sum_as(float mine, float* partials, unsigned* counter, float* sred, float* total) {
+  __shared__ unsigned s_last;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float v = warp_sum(mine);
+  __syncthreads();
+  if (lane == 0) sred[warp] = v;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    float s = 0.f;
+    for (int w = 0; w < NW; ++w) s += sred[w];
+    partials[blockIdx.x] = s;
+    __threadfence();
+    s_last = (atomicAdd(counter, 1u) == gridDim.x - 1) ? 1u : 0u;
+  }
+  __syncthreads();
+  if (!s_last) return false;
+  __threadfence();
+  for (int vw = warp; vw < TV / 32; vw += NW) {
+    float acc = 0.f;
+    for (int i = vw * 32 + lane; i < (int)gridDim.x; i += TV) acc += __ldcg(partials + i);
+    acc = warp_sum(acc);
+    if (lane == 0) sred[vw] = acc;
+  }
+  __syncthreads();
+  float s = 0.f;
+  for (int w = 0; w < TV / 32; ++w) s += sred[w];
+  if (threadIdx.x == 0) *counter = 0u;
+  *total = s;
+  return true;
+}
+
+template <int N, int EPI>
+__global__ void __launch_bounds__(RowWCfg<N>::T, RowOcc<N, 0>::MINB) row_warp_c2r(const __grid_constant__ OpArgs a) {
+  using C = RowWCfg<N>;
+  constexpr int M = C::M, RL = C::RL, RW = C::RW, R0 = C::R0, R1 = C::R1, NSL = C::NSL, NP = C::NP, PITCH = C::PITCH;
+  constexpr int TV = Row2Cfg<N>::T;                      // threads of the older form's CTA
+  constexpr bool HALF = C::HALF;
+  constexpr int J0 = R1;                                 // butterflies per row of the first stage
+  constexpr int V0 = HALF ? R0 / 2 : R0;                 // elements per lane in the first stage
+  static_assert(Plan<M, 0>::stages == 2 && RW * NSL == 32 && (HALF || RW * J0 == 32) && RW * C::NW == RL, "two full stages");
+  static_assert(R1 == 8 || R1 == 16, "skew of the exchange");
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
+  float2* U = reinterpret_cast<float2*>(base);
+  float2* tws = U + M;
+  __shared__ float sred[TV / 32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(base + C::BARS) + 4 * warp;   // [0, 1] spectrum, [2, 3] previous radius
+  unsigned char* bufs = base + C::BUFS + warp * (2 + NP) * C::XBUF;
+
+  constexpr int ntiles = N * N / RL;
+  const int my_count = (int)blockIdx.x < ntiles ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+  const bool has_prev = EPI == EPI_IONIZE && a.has_prev;
+  // first pair of this warp's rows of its CTA's it-th tile
+  auto pair_at = [&](int it) { return ((size_t)(blockIdx.x + it * gridDim.x) * RL + warp * RW) * M; };
+  auto copy_in = [&](const float2* src, unsigned char* dst, uint64_t* bar, uint32_t extra, uint64_t pol) {
+    mbar_expect_tx(bar, (uint32_t)(RW * M * 8) + extra);
+    if (PITCH == M) {
+      bulk_load(dst, src, RW * M * 8, bar, pol);
+    } else {
+#pragma unroll
+      for (int l = 0; l < RW; ++l) bulk_load(dst + l * PITCH * 8, src + l * M, M * 8, bar, pol);
+    }
+  };
+  auto issue = [&](int it) {
+    copy_in(a.cin + pair_at(it), bufs + (it & 1) * C::XBUF, &bars[it & 1], stall_bytes(a.stall, it), l2_policy(a.hint_in));
+  };
+  auto issue_prev = [&](int it) {
+    copy_in(a.prev + pair_at(it), bufs + (2 + it % NP) * C::XBUF, &bars[2 + it % NP], 0u, l2_policy(ES_HINT_EVICT_FIRST));
+  };
+  if (lane == 0) {
+    for (int b = 0; b < 4; ++b) mbar_init(&bars[b], 1);
+    fence_mbar_init();
+    fence_async_smem();
+    for (int it = 0; it < 2 && it < my_count; ++it) issue(it);
+    if (has_prev)
+      for (int it = 0; it < NP && it < my_count; ++it) issue_prev(it);
+  }
+  // U[e] = w^-e for e <= M/2, and -w^(M-e) (the same number as the split of the older form takes it) past it
+  for (int e = threadIdx.x; e < M; e += C::T) {
+    const float2 w = a.tw[e <= M / 2 ? e : M - e];
+    U[e] = e <= M / 2 ? cconj(w) : make_float2(-w.x, -w.y);
+  }
+  for (int i = threadIdx.x; i < C::TW; i += C::T) tws[i] = a.tw[(i % NSL) * (i / NSL + 1) * 2];
+  // previous radius: erfc((dc - d) / denom_prev) * norm_prev >= 1/zeta  <=>  d >= thr_prev
+  float thr_prev = __int_as_float(0x7f800000);
+  if (has_prev) {
+    const float y = a.inv_zeta / a.stats_prev[2];
+    if (y < 2.0f) thr_prev = a.dc - a.denom_prev * erfcinvf(y);
+  }
+  const f32x2 DC = bc2(a.dc), INV = bc2(EPI == EPI_IONIZE ? 1.0f / a.denom : 0.f);
+  f32x2 acc = bc2(0.0f);                                 // two running sums (even, odd voxels)
+  __syncthreads();
+
+  // first stage: lane = (row l0, butterfly j0[, half h]); last stage: lane = (row l, butterfly j)
+  const int l0 = HALF ? lane / (2 * J0) : lane / J0, j0 = HALF ? (lane >> 1) % J0 : lane % J0, h = HALF ? lane & 1 : 0;
+  const int l = lane / NSL, j = lane % NSL;
+  bool ok = true;
+  int it = 0;
+  for (; it < my_count; ++it) {
+    float2* X = reinterpret_cast<float2*>(bufs + (it & 1) * C::XBUF);
+    const size_t pair0 = pair_at(it);
+    ok = __all_sync(0xffffffffu, mbar_wait(&bars[it & 1], (uint32_t)((it >> 1) & 1), a.wait_log2));
+    if (!ok) break;
+    // element r of butterfly j0 is e = j0 + r M / R0; a half-butterfly takes r = 2 k + h
+    float2 v[V0];
+    {
+      const float2* x = X + l0 * PITCH;
+      const int e0 = j0 + h * (M / R0);
+#pragma unroll
+      for (int k = 0; k < V0; ++k) {
+        const int e = e0 + k * (HALF ? 2 : 1) * (M / R0);
+        const float2 own = x[e], u = U[e];
+        const float2 oth = x[k == 0 ? (M - e) & (M - 1) : M - e];
+        const float2 t1 = cmul(u, make_float2(own.x - oth.x, own.y + oth.y));
+        v[k] = make_float2(own.x + oth.x - t1.y, own.y - oth.y + t1.x);
+        if (k == 0 && e == 0) v[k] = make_float2(own.x + own.y, own.x - own.y);   // (X[0], X[N/2]), both real
+      }
+    }
+    if (a.discard_in) {
+      // the intermediate spectrum is dead once copied: drop its lines from L2 unwritten
+      const char* g = reinterpret_cast<const char*>(a.cin + pair0);
+      for (int q = lane; q < RW * M * 8 / 128; q += 32) l2_discard(g + 128 * q);
+    }
+    if constexpr (HALF) {
+      // radix 16 over two lanes: each takes the radix-8 DFT of the even or the odd samples, the odd
+      // ones are turned by w_16^k, and the halves are combined across the pair (Dft<16>)
+      static_assert(R0 == 16, "half butterflies are radix 8");
+      constexpr float c1 = 0.92387953251128674f, s1 = 0.38268343236508978f, rt = 0.70710678118654752f;
+      Dft<8, true>::run(v);
+      if (h) {
+        v[1] = twid<true>(v[1], c1, -s1);
+        v[2] = twid<true>(v[2], rt, -rt);
+        v[3] = twid<true>(v[3], s1, -c1);
+        v[4] = rot<true>(v[4]);
+        v[5] = twid<true>(v[5], -s1, -c1);
+        v[6] = twid<true>(v[6], -rt, -rt);
+        v[7] = twid<true>(v[7], -c1, -s1);
+      }
+      const float sg = h ? -1.0f : 1.0f;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {                      // even lane: e + o; odd lane: e - o (outputs 8 + k)
+        const float ox = __shfl_xor_sync(0xffffffffu, v[k].x, 1), oy = __shfl_xor_sync(0xffffffffu, v[k].y, 1);
+        v[k] = make_float2(fmaf(v[k].x, sg, ox), fmaf(v[k].y, sg, oy));
+      }
+    } else {
+      Dft<R0, true>::run(v);
+    }
+    __syncwarp();                                        // every lane has read its rows
+    // exchange: output r of butterfly j0 goes to slot j0 R0 + (r ^ j0)
+    {
+      float2* x = X + l0 * PITCH + j0 * R0 + h * V0;
+#pragma unroll
+      for (int k = 0; k < V0; ++k) x[k ^ (HALF ? (j0 & 7) : j0)] = v[k];
+    }
+    __syncwarp();
+    float2 z[R1];
+    {
+      const float2* x = X + l * PITCH;
+#pragma unroll
+      for (int r = 0; r < R1; ++r) z[r] = x[r * R0 + (j ^ r)];
+    }
+    // the buffer takes the tile after next
+    fence_async_smem();
+    __syncwarp();
+    if (lane == 0 && it + 2 < my_count) issue(it + 2);
+#pragma unroll
+    for (int r = 1; r < R1; ++r) {
+      const float2 w = tws[(r - 1) * NSL + j];
+      z[r] = twid<true>(z[r], w.x, w.y);
+    }
+    Dft<R1, true>::run(z);
+    // element p = j + r NSL of row l
+    const size_t row0 = pair0 + (size_t)l * M;
+    if (EPI == EPI_STORE) {
+#pragma unroll
+      for (int r = 0; r < R1; ++r) a.rout[row0 + j + r * NSL] = z[r];
+      continue;
+    }
+    // the erfc sum first: the chains are independent and overlap
+    {
+      f32x2 e[R1];
+#pragma unroll
+      for (int r = 0; r < R1; ++r) e[r] = erfc_sum_pair(mul2(sub2(DC, pk2(z[r].x, z[r].y)), INV));
+#pragma unroll
+      for (int r = 0; r < R1; ++r) acc = add2(acc, e[r]);
+    }
+    // the previous radius' delta_R of this lane's elements
+    const float2* pv = reinterpret_cast<const float2*>(bufs + (2 + it % NP) * C::XBUF) + l * PITCH + j;
+    if (has_prev) {
+      ok = __all_sync(0xffffffffu, mbar_wait(&bars[2 + it % NP], (uint32_t)((it / NP) & 1), a.wait_log2));
+      if (!ok) break;
+    }
+    if (a.marker) {
+      // centre mode: whether a cell passed at an earlier radius travels in the lowest mantissa bit of
+      // delta_R (a change of at most one unit in the last place), so the next radius carries it on
+#pragma unroll
+      for (int r = 0; r < R1; ++r) {
+        unsigned fx = 0u, fy = 0u;
+        if (has_prev) {
+          const float2 pp = pv[r * NSL];
+          fx = (__float_as_uint(pp.x) & 1u) | (pp.x >= thr_prev ? 1u : 0u);
+          fy = (__float_as_uint(pp.y) & 1u) | (pp.y >= thr_prev ? 1u : 0u);
+        }
+        __stcs(a.rout + row0 + j + r * NSL, make_float2(__uint_as_float((__float_as_uint(z[r].x) & ~1u) | fx),
+                                                       __uint_as_float((__float_as_uint(z[r].y) & ~1u) | fy)));
+      }
+    } else {
+      // sphere mode: delta_R as it is, and the centres' bitmap, 8 consecutive pairs per store
+      unsigned cnt = 0u;
+#pragma unroll
+      for (int r = 0; r < R1; ++r) {
+        __stcs(a.rout + row0 + j + r * NSL, z[r]);
+        if (has_prev) {
+          const float2 pp = pv[r * NSL];
+          const unsigned bx = __ballot_sync(0xffffffffu, pp.x >= thr_prev);
+          const unsigned by = __ballot_sync(0xffffffffu, pp.y >= thr_prev);
+          cnt += __popc(bx) + __popc(by);
+          if ((lane & 7) == 0) put_centres<N>(a.centres, row0 / M, j + r * NSL, bx >> lane, by >> lane);
+        }
+      }
+      if (lane == 0 && cnt) atomicAdd(a.centre_count, cnt);
+    }
+    if (has_prev) {
+      fence_async_smem();
+      __syncwarp();
+      if (lane == 0 && it + NP < my_count) issue_prev(it + NP);
+    }
+  }
+  if (!ok) {
+    // a wait ran out: record it; the copies in flight land (bounded waits) before the CTA leaves
+    if (lane == 0) {
+      atomicOr(a.err, ES_DEV_ERR_TIMEOUT);
+      for (int q = it; q < it + 3 && q < my_count; ++q) mbar_wait(&bars[q & 1], (uint32_t)((q >> 1) & 1), a.wait_log2);
+      if (has_prev)
+        for (int q = it; q < it + NP && q < my_count; ++q)
+          mbar_wait(&bars[2 + q % NP], (uint32_t)((q / NP) & 1), a.wait_log2);
+    }
+    __syncwarp();
+  }
+  if (EPI == EPI_IONIZE) {
+    float total;
+    const float2 acc2 = upk2(acc);
+    if (grid_sum_as<TV, C::NW>(acc2.x + acc2.y, a.partials, a.counter, sred, &total) && threadIdx.x == 0) {
+      const float mean = total / ((float)N * (float)N * (float)N);
+      a.stats_out[0] = total;
+      a.stats_out[1] = mean;
+      a.stats_out[2] = a.normalize ? a.fc_mean / mean : 1.f;
+    }
+  }
+}
+
+}  // namespace es
