@@ -195,7 +195,7 @@ __global__ void __launch_bounds__(ColWSmem<N, MODE>::T, 1) col_warp(const __grid
   constexpr bool INV = MODE == COL_Z_INV_FILTER || MODE == COL_Y_INV || MODE == COL_Z_INV;
   constexpr bool ZPASS = ColWSeq<N, MODE>::ZPASS;
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  unsigned char* base = align_smem<1024>(smem_raw);
   uint64_t* full = reinterpret_cast<uint64_t*>(base + NBUF * SM::tile);
   uint64_t* done = full + NBUF;
   float2* tws = reinterpret_cast<float2*>(done + NBUF);

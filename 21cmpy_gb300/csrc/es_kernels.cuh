@@ -199,6 +199,12 @@ __device__ __forceinline__ float ex2_approx(float x) {
   return y;
 }
 
+__device__ __forceinline__ float rcp_approx(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
 // erfc_sum_term for two arguments at once on packed pairs (the same Numerical Recipes erfcc).
 // log2(e) is folded into the polynomial and the constant so the exponential is one ex2 of
 // (t P(t) - 1.26551223 - z^2) log2(e); z^2 = hi + lo is split exactly as above.  For x < 0 the
@@ -207,9 +213,8 @@ __device__ __forceinline__ f32x2 erfc_sum_pair(f32x2 xv) {
   constexpr float L2E = 1.4426950408889634f;
   const float2 x = upk2(xv);
   const float z0 = fabsf(x.x), z1 = fabsf(x.y);
-  const f32x2 Z = pk2(z0, z1), NZ = pk2(-z0, -z1);
-  const float2 d = upk2(fma2(Z, bc2(0.5f), bc2(1.0f)));
-  const f32x2 T = pk2(__fdividef(1.0f, d.x), __fdividef(1.0f, d.y));
+  const float2 d = upk2(fma2(pk2(z0, z1), bc2(0.5f), bc2(1.0f)));
+  const f32x2 T = pk2(rcp_approx(d.x), rcp_approx(d.y));   // divisors in [1, 11]: normal numbers
   f32x2 P = bc2(0.17087277f * L2E);
   P = fma2(P, T, bc2(-0.82215223f * L2E));
   P = fma2(P, T, bc2(1.48851587f * L2E));
@@ -219,8 +224,8 @@ __device__ __forceinline__ f32x2 erfc_sum_pair(f32x2 xv) {
   P = fma2(P, T, bc2(0.09678418f * L2E));
   P = fma2(P, T, bc2(0.37409196f * L2E));
   P = fma2(P, T, bc2(1.00002368f * L2E));
-  const f32x2 H = mul2(Z, Z);                        // hi = z^2 rounded
-  const f32x2 NLO = fma2(NZ, Z, H);                  // hi - z^2 = -lo exactly
+  const f32x2 H = mul2(xv, xv);                      // hi = z^2 rounded
+  const f32x2 NLO = fma2(mul2(xv, bc2(-1.0f)), xv, H);   // hi - z^2 = -lo exactly
   f32x2 E = fma2(T, P, bc2(-1.26551223f * L2E));
   E = fma2(H, bc2(-L2E), E);
   const float2 e = upk2(E);

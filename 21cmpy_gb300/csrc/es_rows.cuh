@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(RowTile<N, V>::T, RowOcc<N, V>::MINB) row2_c2r
   constexpr unsigned GMASK = G == 32 ? 0xffffffffu : ((1u << G) - 1u);
   static_assert((RL * N) % 64 == 0 && (RL * M) % 32 == 0, "row tiles must hold whole 64-voxel flag pairs");
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
+  unsigned char* base = align_smem<128>(smem_raw);
   float2* const S0 = reinterpret_cast<float2*>(base);
   float2* const S1 = reinterpret_cast<float2*>(base + SM::stage);
   float2* A = reinterpret_cast<float2*>(base + 2 * SM::stage);
@@ -404,7 +404,7 @@ __global__ void __launch_bounds__(RowTile<N, V>::T, RowOcc<N, V>::MINB) row2_r2c
   constexpr int M = N / 2, RL = RowTile<N, V>::RL, T = RowTile<N, V>::T, ES = RL + 1;
   using SM = Row2Smem<N, false, V>;
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
+  unsigned char* base = align_smem<128>(smem_raw);
   float2* const S0 = reinterpret_cast<float2*>(base);
   float2* const S1 = reinterpret_cast<float2*>(base + SM::stage);
   float2* A = reinterpret_cast<float2*>(base + 2 * SM::stage);

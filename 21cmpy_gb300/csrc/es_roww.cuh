@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(RowWCfg<N>::T, RowOcc<N, 0>::MINB) row_warp_c2
   static_assert(Plan<M, 0>::stages == 2 && RW * NSL == 32 && (HALF || RW * J0 == 32) && RW * C::NW == RL, "two full stages");
   static_assert(R1 == 8 || R1 == 16, "skew of the exchange");
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
+  unsigned char* base = align_smem<128>(smem_raw);
   float2* U = reinterpret_cast<float2*>(base);
   float2* tws = U + M;
   __shared__ float sred[TV / 32];
@@ -100,9 +100,10 @@ __global__ void __launch_bounds__(RowWCfg<N>::T, RowOcc<N, 0>::MINB) row_warp_c2
   constexpr int ntiles = N * N / RL;
   const int my_count = (int)blockIdx.x < ntiles ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
   const bool has_prev = EPI == EPI_IONIZE && a.has_prev;
-  // first pair of this warp's rows of its CTA's it-th tile
-  auto pair_at = [&](int it) { return ((size_t)(blockIdx.x + it * gridDim.x) * RL + warp * RW) * M; };
-  auto copy_in = [&](const float2* src, unsigned char* dst, uint64_t* bar, uint32_t extra, uint64_t pol) {
+  // first pair of this warp's rows of its CTA's it-th tile (at most 512^3 / 2 pairs: 32 bits)
+  auto pair_at = [&](int it) { return ((blockIdx.x + it * gridDim.x) * RL + warp * RW) * M; };
+  auto copy_in = [&](const float2* src, unsigned char* dst, uint64_t* bar, uint32_t extra, int hint) {
+    const uint64_t pol = l2_policy(hint);
     mbar_expect_tx(bar, (uint32_t)(RW * M * 8) + extra);
     if (PITCH == M) {
       bulk_load(dst, src, RW * M * 8, bar, pol);
@@ -112,10 +113,10 @@ __global__ void __launch_bounds__(RowWCfg<N>::T, RowOcc<N, 0>::MINB) row_warp_c2
     }
   };
   auto issue = [&](int it) {
-    copy_in(a.cin + pair_at(it), bufs + (it & 1) * C::XBUF, &bars[it & 1], stall_bytes(a.stall, it), l2_policy(a.hint_in));
+    copy_in(a.cin + pair_at(it), bufs + (it & 1) * C::XBUF, &bars[it & 1], stall_bytes(a.stall, it), a.hint_in);
   };
   auto issue_prev = [&](int it) {
-    copy_in(a.prev + pair_at(it), bufs + (2 + it % NP) * C::XBUF, &bars[2 + it % NP], 0u, l2_policy(ES_HINT_EVICT_FIRST));
+    copy_in(a.prev + pair_at(it), bufs + (2 + it % NP) * C::XBUF, &bars[2 + it % NP], 0u, ES_HINT_EVICT_FIRST);
   };
   if (lane == 0) {
     for (int b = 0; b < 4; ++b) mbar_init(&bars[b], 1);
@@ -148,7 +149,7 @@ __global__ void __launch_bounds__(RowWCfg<N>::T, RowOcc<N, 0>::MINB) row_warp_c2
   int it = 0;
   for (; it < my_count; ++it) {
     float2* X = reinterpret_cast<float2*>(bufs + (it & 1) * C::XBUF);
-    const size_t pair0 = pair_at(it);
+    const uint32_t pair0 = pair_at(it);
     ok = __all_sync(0xffffffffu, mbar_wait(&bars[it & 1], (uint32_t)((it >> 1) & 1), a.wait_log2));
     if (!ok) break;
     // element r of butterfly j0 is e = j0 + r M / R0; a half-butterfly takes r = 2 k + h
@@ -168,8 +169,10 @@ __global__ void __launch_bounds__(RowWCfg<N>::T, RowOcc<N, 0>::MINB) row_warp_c2
     }
     if (a.discard_in) {
       // the intermediate spectrum is dead once copied: drop its lines from L2 unwritten
-      const char* g = reinterpret_cast<const char*>(a.cin + pair0);
-      for (int q = lane; q < RW * M * 8 / 128; q += 32) l2_discard(g + 128 * q);
+      const float2* g = a.cin + pair0 + 16 * lane;
+#pragma unroll
+      for (int q = 0; q < RW * M / 16; q += 32)
+        if (q + lane < RW * M / 16) l2_discard(g + 16 * q);
     }
     if constexpr (HALF) {
       // radix 16 over two lanes: each takes the radix-8 DFT of the even or the odd samples, the odd
@@ -220,10 +223,11 @@ __global__ void __launch_bounds__(RowWCfg<N>::T, RowOcc<N, 0>::MINB) row_warp_c2
     }
     Dft<R1, true>::run(z);
     // element p = j + r NSL of row l
-    const size_t row0 = pair0 + (size_t)l * M;
+    const uint32_t row0 = pair0 + l * M;
+    float2* out = a.rout + row0 + j;
     if (EPI == EPI_STORE) {
 #pragma unroll
-      for (int r = 0; r < R1; ++r) a.rout[row0 + j + r * NSL] = z[r];
+      for (int r = 0; r < R1; ++r) out[r * NSL] = z[r];
       continue;
     }
     // the erfc sum first: the chains are independent and overlap
@@ -245,21 +249,21 @@ __global__ void __launch_bounds__(RowWCfg<N>::T, RowOcc<N, 0>::MINB) row_warp_c2
       // delta_R (a change of at most one unit in the last place), so the next radius carries it on
 #pragma unroll
       for (int r = 0; r < R1; ++r) {
-        unsigned fx = 0u, fy = 0u;
+        unsigned fx = 0u, fy = 0u;                       // flags in bit 0
         if (has_prev) {
           const float2 pp = pv[r * NSL];
-          fx = (__float_as_uint(pp.x) & 1u) | (pp.x >= thr_prev ? 1u : 0u);
-          fy = (__float_as_uint(pp.y) & 1u) | (pp.y >= thr_prev ? 1u : 0u);
+          fx = pp.x >= thr_prev ? 1u : __float_as_uint(pp.x);
+          fy = pp.y >= thr_prev ? 1u : __float_as_uint(pp.y);
         }
-        __stcs(a.rout + row0 + j + r * NSL, make_float2(__uint_as_float((__float_as_uint(z[r].x) & ~1u) | fx),
-                                                       __uint_as_float((__float_as_uint(z[r].y) & ~1u) | fy)));
+        __stcs(out + r * NSL, make_float2(__uint_as_float((__float_as_uint(z[r].x) & ~1u) | (fx & 1u)),
+                                         __uint_as_float((__float_as_uint(z[r].y) & ~1u) | (fy & 1u))));
       }
     } else {
       // sphere mode: delta_R as it is, and the centres' bitmap, 8 consecutive pairs per store
       unsigned cnt = 0u;
 #pragma unroll
       for (int r = 0; r < R1; ++r) {
-        __stcs(a.rout + row0 + j + r * NSL, z[r]);
+        __stcs(out + r * NSL, z[r]);
         if (has_prev) {
           const float2 pp = pv[r * NSL];
           const unsigned bx = __ballot_sync(0xffffffffu, pp.x >= thr_prev);

@@ -13,6 +13,12 @@ constexpr int kWaitLog2 = 26;             // default: 2^26 mbarrier polls before
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
+// The dynamic shared memory from its first multiple of A bytes.  An offset, not a rounded pointer: through
+// an integer the compiler loses that the pointer is to shared memory and every access becomes a
+// generic one, with 64-bit addresses (row C2R + ionise at 256^3: 42.2 us against 39.5 us, z inverse 24.8 against 23.1).
+template <int A> __device__ __forceinline__ unsigned char* align_smem(unsigned char* p) {
+  return p + ((0u - smem_u32(p)) & (uint32_t)(A - 1));
+}
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
 }
@@ -238,7 +244,7 @@ __global__ void __launch_bounds__(ColTile<N, V>::T, ColTile<N, V>::MINB) col_tma
 
   extern __shared__ __align__(128) unsigned char smem_raw[];
   // TMA destinations must be 128-byte aligned: align the base explicitly (128 bytes of slack)
-  unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
+  unsigned char* base = align_smem<128>(smem_raw);
   float2* S0 = reinterpret_cast<float2*>(base);
   float2* S1 = S0 + N * TI;
   float2* W = S1 + N * TI;
