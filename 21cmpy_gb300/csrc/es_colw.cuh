@@ -227,9 +227,13 @@ __global__ void __launch_bounds__(ColWSmem<N, MODE>::T, 1) col_warp(const __grid
     }
     fence_mbar_init();
     fence_async_smem();
-    for (int it = 0; it < NBUF && it < seq.count; ++it) load(it);
   }
   F::load_twiddles(tws, a.tw, threadIdx.x, SM::T);
+  if (!a.early) pdl_wait();
+  if (threadIdx.x == 32 * SM::NW) {
+    for (int it = 0; it < NBUF && it < seq.count; ++it) load(it);
+    if (!a.early) pdl_trigger();
+  }
   __syncthreads();
 
   if (warp == SM::NW) {
@@ -238,6 +242,10 @@ __global__ void __launch_bounds__(ColWSmem<N, MODE>::T, 1) col_warp(const __grid
       int loaded = seq.count < NBUF ? seq.count : NBUF;
       for (int it = 0; it < seq.count; ++it) {
         if (!colw_wait(&done[it % NBUF], (uint32_t)((it / NBUF) & 1), a, abort)) break;
+        if (a.early && it == 0) {
+          pdl_wait();
+          pdl_trigger();
+        }
         const ColWTile t = seq.at(it);
         const unsigned char* src = base + (it % NBUF) * SM::tile;
         const uint64_t pol = l2_policy(a.hint_out);
@@ -259,6 +267,7 @@ __global__ void __launch_bounds__(ColWSmem<N, MODE>::T, 1) col_warp(const __grid
       if (*abort)
         for (int it = loaded > NBUF ? loaded - NBUF : 0; it < loaded; ++it)
           mbar_wait(&full[it % NBUF], (uint32_t)((it / NBUF) & 1), a.wait_log2);
+      if (a.early) pdl_wait();                           // also where this CTA has stored nothing
       bulk_wait0();
     }
     return;

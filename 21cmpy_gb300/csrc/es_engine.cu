@@ -209,6 +209,8 @@ __global__ void __launch_bounds__(T) final_kernel(const float2* dR, const uint32
                                                   float2* out, float* partials, unsigned* counter,
                                                   float* nf, float inv_n3) {
   __shared__ float sred[T / 32];
+  es::pdl_wait();
+  es::pdl_trigger();
   const es::f32x2 NORM = es::bc2(stats[2]), DC = es::bc2(dc), INV = es::bc2(1.0f / denom);
   float acc = 0.f;
   for (long p = blockIdx.x * (long)T + threadIdx.x; p < pairs; p += (long)gridDim.x * T) {
@@ -238,6 +240,8 @@ __global__ void __launch_bounds__(T) delta_T_kernel(const float2* xH, const floa
                                                     float c, float2* dT, float* partials,
                                                     unsigned* counter, float* ave, float inv_n3) {
   __shared__ float sred[T / 32];
+  es::pdl_wait();
+  es::pdl_trigger();
   float acc = 0.f;
   for (long p = blockIdx.x * (long)T + threadIdx.x; p < pairs; p += (long)gridDim.x * T) {
     const float2 x = xH[p], d = delta[p];
@@ -546,6 +550,27 @@ void set_maps(es::OpArgs& a, const es_plan* p, int in, int out, bool z, bool col
   a.tm_out_nyq = mo->nyq;
 }
 
+// Whether a plan's kernels are launched with programmatic stream serialisation (es::pdl_wait).  Up to 256^3
+// a pass lasts 4-40 us, of which launch and set-up are a good part.  At 512^3 it lasts 200-260 us and is
+// bound by DRAM, which likes all CTAs to walk the spectrum in step: CTAs that start as the previous
+// kernel's leave lose more by that than the launch gaps cost (whole box 28.8 ms without, 31.2 with).  The
+// synchronous passes have no pdl_wait.
+bool uses_pdl(const es_plan* p) { return p->col_variant == 1 && p->n <= 256; }
+
+template <class... P, class... A>
+cudaError_t launch_pdl(bool pdl, void (*kernel)(P...), int grid, int threads, cudaStream_t s, A... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.stream = s;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = pdl ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // Records the start event of a timed launch; returns the slot or -1 when timing is off/full.
 int prof_begin(es_plan* p, int op, cudaStream_t s) {
   if (p->prof_events.empty()) return -1;
@@ -561,6 +586,7 @@ void prof_end(es_plan* p, int slot, cudaStream_t s) {
 
 int run_op(es_plan* p, int op, es::OpArgs a, int grid, cudaStream_t s) {
   a.grid = grid;
+  a.pdl = uses_pdl(p);
   a.stall = (p->stall == ES_STALL_COL_Z_INV && op == es::OP_COL_Z_INV_FILTER) ||
             (p->stall == ES_STALL_ROW_C2R && op == es::OP_ROW_C2R_IONIZE) ||
             (p->stall == ES_STALL_ROW_R2C && op == es::OP_ROW_R2C_SCALE);
@@ -828,6 +854,9 @@ int es_ionize(es_plan* p, const es_ionize_params* prm, float* out, float* nf, vo
   const TBuf tb[2] = {{p->T, p->Tnyq, SPEC_T}, {p->T2, p->Tnyq2, SPEC_T2}};
   const bool cw = uses_col_warp(p, true);
   const bool ovl = p->overlap != 0 && nr > 1;
+  // one stream, and only kernels with a pdl_wait between: what a kernel before the preceding one wrote is
+  // complete (es::pdl_wait)
+  const bool serial = !ovl && uses_pdl(p);
   auto capped = [&](int grid, int per_sm) { return (ovl && per_sm > 0 && grid > p->sms * per_sm) ? p->sms * per_sm : grid; };
   const int g_z = capped(grid_col_z(p, false), p->col_per_sm), g_y = capped(grid_col_y(p), p->col_per_sm);
   const int g_row = capped(grid_row(p, true), p->row_per_sm);
@@ -846,6 +875,7 @@ int es_ionize(es_plan* p, const es_ionize_params* prm, float* out, float* nf, vo
     a.inv_n3 = inv_n3;
     a.hint_in = p->l2_hints ? es::ES_HINT_EVICT_FIRST : es::ES_HINT_NORMAL;
     a.hint_out = keep;
+    a.early = serial && r > 0;      // the input spectrum is the forward transform's
     set_maps(a, p, SPEC_X, t.spec, true, cw);
     if (int e = run_op(p, es::OP_COL_Z_INV_FILTER, a, g_z, cs)) return e;
     a = base_args(p);
@@ -878,6 +908,7 @@ int es_ionize(es_plan* p, const es_ionize_params* prm, float* out, float* nf, vo
     a.normalize = prm->normalize_mean;
     a.hint_in = p->l2_hints ? es::ES_HINT_EVICT_FIRST : es::ES_HINT_NORMAL;
     a.discard_in = p->l2_hints;
+    a.early = serial;               // the previous radius' row pass came before this radius' column passes
     if (int e = run_op(p, es::OP_ROW_C2R_IONIZE, a, g_row, s)) return e;
     if (prm->update == 1 && r > 0) {
       const int ps = prof_begin(p, ES_PROF_PAINT, s);
@@ -921,12 +952,12 @@ int es_ionize(es_plan* p, const es_ionize_params* prm, float* out, float* nf, vo
     }
   }
   slot = prof_begin(p, ES_PROF_FINAL, s);
-  final_kernel<256><<<grid_elem(p), 256, 0, s>>>(
-      reinterpret_cast<const float2*>(p->dR[(nr - 1) & 1]), p->flags, marker, (long)(N3 / 2), prm->delta_c,
-      prm->radii[nr - 1].denom, p->stats + (size_t)(nr - 1) * kStatsStride, prm->zeta, inv_zeta,
-      prm->output, reinterpret_cast<float2*>(out), p->partials, p->counters, nf, inv_n3);
+  const cudaError_t le = launch_pdl(
+      uses_pdl(p), final_kernel<256>, grid_elem(p), 256, s, reinterpret_cast<const float2*>(p->dR[(nr - 1) & 1]), p->flags, marker,
+      (long)(N3 / 2), prm->delta_c, prm->radii[nr - 1].denom, p->stats + (size_t)(nr - 1) * kStatsStride, prm->zeta,
+      inv_zeta, prm->output, reinterpret_cast<float2*>(out), p->partials, p->counters, nf, inv_n3);
   prof_end(p, slot, s);
-  ES_CUDA(cudaGetLastError());
+  ES_CUDA(le);
   return ES_OK;
 }
 
@@ -935,11 +966,12 @@ int es_delta_T(es_plan* p, const float* xH, const float* delta, float c, float* 
   DeviceGuard g(p->device);
   const size_t N3 = (size_t)p->n * p->n * p->n;
   const int slot = prof_begin(p, ES_PROF_DELTA_T, (cudaStream_t)stream);
-  delta_T_kernel<256><<<grid_elem(p), 256, 0, (cudaStream_t)stream>>>(
-      reinterpret_cast<const float2*>(xH), reinterpret_cast<const float2*>(delta), (long)(N3 / 2), c,
-      reinterpret_cast<float2*>(dT), p->partials, p->counters, ave, (float)(1.0 / (double)N3));
+  const cudaError_t le = launch_pdl(
+      uses_pdl(p), delta_T_kernel<256>, grid_elem(p), 256, (cudaStream_t)stream, reinterpret_cast<const float2*>(xH),
+      reinterpret_cast<const float2*>(delta), (long)(N3 / 2), c, reinterpret_cast<float2*>(dT), p->partials, p->counters,
+      ave, (float)(1.0 / (double)N3));
   prof_end(p, slot, (cudaStream_t)stream);
-  ES_CUDA(cudaGetLastError());
+  ES_CUDA(le);
   return ES_OK;
 }
 

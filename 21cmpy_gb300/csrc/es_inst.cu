@@ -36,8 +36,17 @@ static cudaError_t launch(int smem, const OpArgs& a, int threads, cudaStream_t s
     configured |= bit;
   }
   const int grid = a.grid < resident[dev & 31] ? a.grid : resident[dev & 31];
-  Kernel<<<grid, threads, smem, s>>>(a);
-  return cudaGetLastError();
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = (size_t)smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = a.pdl ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, Kernel, a);
 }
 
 template <int N, int MODE, int RS>

@@ -142,9 +142,12 @@ __global__ void __launch_bounds__(RowTile<N, V>::T, RowOcc<N, V>::MINB) row2_c2r
     for (int b = 0; b < 4; ++b) mbar_init(&bars[b], 1);
     fence_mbar_init();
     fence_async_smem();
-    for (int s = 0; s < 2 && s < my_count; ++s) issue(s, s);
   }
   for (int i = threadIdx.x; i < N; i += T) tw[i] = a.tw[i];
+  pdl_wait();
+  if (threadIdx.x == 0)
+    for (int s = 0; s < 2 && s < my_count; ++s) issue(s, s);
+  pdl_trigger();
   // previous radius: erfc((dc - d) / denom_prev) * norm_prev >= 1/zeta  <=>  d >= thr_prev
   float thr_prev = __int_as_float(0x7f800000);
   if (has_prev) {
@@ -427,9 +430,12 @@ __global__ void __launch_bounds__(RowTile<N, V>::T, RowOcc<N, V>::MINB) row2_r2c
     mbar_init(&bars[1], 1);
     fence_mbar_init();
     fence_async_smem();
-    for (int s = 0; s < 2 && s < my_count; ++s) issue(s, s);
   }
   for (int i = threadIdx.x; i < N; i += T) tw[i] = a.tw[i];
+  pdl_wait();
+  if (threadIdx.x == 0)
+    for (int s = 0; s < 2 && s < my_count; ++s) issue(s, s);
+  pdl_trigger();
   float sc = a.scale, sh = 0.f;
   if (PRO == PRO_PK) {
     const float ave = *a.ave;

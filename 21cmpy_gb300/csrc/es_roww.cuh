@@ -122,8 +122,7 @@ __global__ void __launch_bounds__(RowWCfg<N>::T, RowOcc<N, 0>::MINB) row_warp_c2
     for (int b = 0; b < 4; ++b) mbar_init(&bars[b], 1);
     fence_mbar_init();
     fence_async_smem();
-    for (int it = 0; it < 2 && it < my_count; ++it) issue(it);
-    if (has_prev)
+    if (has_prev && a.early)
       for (int it = 0; it < NP && it < my_count; ++it) issue_prev(it);
   }
   // U[e] = w^-e for e <= M/2, and -w^(M-e) (the same number as the split of the older form takes it) past it
@@ -132,6 +131,13 @@ __global__ void __launch_bounds__(RowWCfg<N>::T, RowOcc<N, 0>::MINB) row_warp_c2
     U[e] = e <= M / 2 ? cconj(w) : make_float2(-w.x, -w.y);
   }
   for (int i = threadIdx.x; i < C::TW; i += C::T) tws[i] = a.tw[(i % NSL) * (i / NSL + 1) * 2];
+  pdl_wait();
+  if (lane == 0) {
+    for (int it = 0; it < 2 && it < my_count; ++it) issue(it);
+    if (has_prev && !a.early)
+      for (int it = 0; it < NP && it < my_count; ++it) issue_prev(it);
+  }
+  pdl_trigger();
   // previous radius: erfc((dc - d) / denom_prev) * norm_prev >= 1/zeta  <=>  d >= thr_prev
   float thr_prev = __int_as_float(0x7f800000);
   if (has_prev) {

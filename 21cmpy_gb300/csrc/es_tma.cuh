@@ -264,10 +264,14 @@ __global__ void __launch_bounds__(ColTile<N, V>::T, ColTile<N, V>::MINB) col_tma
     mbar_init(&bars[1], 1);
     fence_mbar_init();
     fence_async_smem();
-    for (int s = 0; s < 2 && s < my_count; ++s)
-      issue_tile_load<N, MODE, V>(a, seq.at(s, &reuse_w), s ? S1 : S0, &bars[s], stall_bytes(a.stall, s));
   }
   for (int i = threadIdx.x; i < N; i += T) tw[i] = a.tw[i];
+  if (!a.early) pdl_wait();
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < 2 && s < my_count; ++s)
+      issue_tile_load<N, MODE, V>(a, seq.at(s, &reuse_w), s ? S1 : S0, &bars[s], stall_bytes(a.stall, s));
+    if (!a.early) pdl_trigger();
+  }
   if (MODE == COL_Z_FWD_PK) {
     for (int i = threadIdx.x; i < (T / 32) * PK_MAX_BINS * 3; i += T) bins[i] = 0.f;
     for (int i = threadIdx.x; i < a.nbins; i += T) sthr[i] = a.thr[i];
@@ -366,10 +370,19 @@ __global__ void __launch_bounds__(ColTile<N, V>::T, ColTile<N, V>::MINB) col_tma
       }
       fence_async_smem();
       __syncthreads();
-      if (threadIdx.x == 0) issue_tile_store<N, MODE, V>(a, t, out);
+      if (threadIdx.x == 0) {
+        if (a.early && it == 0) {
+          pdl_wait();
+          pdl_trigger();
+        }
+        issue_tile_store<N, MODE, V>(a, t, out);
+      }
     }
   }
-  if (threadIdx.x == 0) bulk_wait0();
+  if (threadIdx.x == 0) {
+    if (a.early) pdl_wait();                             // also where this CTA has stored nothing
+    bulk_wait0();
+  }
 
   if (MODE == COL_Z_FWD_PK) pk_finish<T>(bins, a);
 }
