@@ -84,6 +84,11 @@ _PROTOS = {
                                     C.c_void_p, C.c_void_p]),
     "es_fft_r2c": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]),
     "es_fft_c2r": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]),
+    "es_fft_c2r_scaled": (C.c_int, [C.c_void_p, C.c_void_p, C.c_float, C.c_void_p, C.c_void_p]),
+    "es_fft_forward": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p]),
+    "es_fft_plan_bytes": (C.c_size_t, [C.c_int, C.c_int]),
+    "es_fft_plan_create": (C.c_int, [C.c_int, C.c_double, C.c_int, C.c_void_p, C.c_void_p, C.c_size_t, C.c_void_p,
+                                     C.POINTER(C.c_void_p)]),
     "es_profile_enable": (C.c_int, [C.c_void_p, C.c_int]),
     "es_profile_reset": (C.c_int, [C.c_void_p]),
     "es_profile_read": (C.c_int, [C.c_void_p, C.POINTER(C.c_float), C.POINTER(C.c_int), C.c_int]),
@@ -124,6 +129,8 @@ _PROTOS = {
                               C.c_void_p, C.c_void_p]),
     "ic_shape": (C.c_int, [C.c_int, C.c_float, C.c_void_p, C.c_int, C.c_int, C.c_float, C.c_int, C.c_void_p,
                            C.c_void_p]),
+    "ic_sampled_fields": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_float, C.c_int, C.c_int, C.c_int,
+                                    C.c_float, C.POINTER(C.c_void_p), C.c_void_p]),
     "ic_subsample": (C.c_int, [C.c_int, C.c_int, C.c_float, C.c_float, C.c_void_p, C.c_void_p, C.c_void_p]),
     "ic_last_error": (C.c_int, [C.c_char_p, C.c_int]),
     "es_last_error": (C.c_int, [C.c_char_p, C.c_int]),

@@ -76,7 +76,7 @@ struct RadDev {
 
 // TMA descriptors of one spectrum: main array with z-pass and y-pass boxes, Nyquist plane
 struct MapSet { CUtensorMap z, y, nyq; };
-enum { SPEC_X = 0, SPEC_T = 1, SPEC_T2 = 2 };
+enum { SPEC_X = 0, SPEC_T = 1, SPEC_T2 = 2, kMaxSpectra = 4 };
 
 struct es_plan {
   int n = 0, m = 0, device = 0, sms = 0, max_radii = 0, k2n = 0;
@@ -110,7 +110,10 @@ struct es_plan {
   int prof_dropped = 0;
   // TMA descriptors of the three spectra for the TMA column passes (tm, tile width of col_tile) and for
   // the warp-per-columns form (tms, swizzled); index SPEC_X, SPEC_T, SPEC_T2
-  MapSet tm[3], tms[3];
+  MapSet tm[kMaxSpectra], tms[kMaxSpectra];
+  float2 *spec[kMaxSpectra] = {}, *spec_nyq[kMaxSpectra] = {};   // the spectra themselves
+  int nspec = 3;
+  bool fft_only = false;            // es_fft_plan_create: spectra in the caller's memory, transforms alone
   // overlapped radii: a second intermediate spectrum so the column passes of radius r + 1 run on
   // the plan's own stream while the row pass of radius r runs on the caller's
   float2* T2 = nullptr;
@@ -497,13 +500,11 @@ int make_nyq_map(CUtensorMap* m, void* base, int n, int ti, CUtensorMapSwizzle s
 
 // TMA descriptors of the plan's spectra for a column tile width
 int encode_set(es_plan* p, MapSet* set, int ti, CUtensorMapSwizzle swizzle) {
-  float2* const main[3] = {p->X, p->T, p->T2};
-  float2* const nyq[3] = {p->Xnyq, p->Tnyq, p->Tnyq2};
-  for (int i = 0; i < 3; ++i) {
+  for (int i = 0; i < p->nspec; ++i) {
     int rc = 0;
-    if ((rc = make_main_map(&set[i].z, main[i], p->n, ti, true, swizzle)) ||
-        (rc = make_main_map(&set[i].y, main[i], p->n, ti, false, swizzle)) ||
-        (rc = make_nyq_map(&set[i].nyq, nyq[i], p->n, ti, swizzle)))
+    if ((rc = make_main_map(&set[i].z, p->spec[i], p->n, ti, true, swizzle)) ||
+        (rc = make_main_map(&set[i].y, p->spec[i], p->n, ti, false, swizzle)) ||
+        (rc = make_nyq_map(&set[i].nyq, p->spec_nyq[i], p->n, ti, swizzle)))
       return rc;
   }
   return ES_OK;
@@ -629,11 +630,13 @@ int reuse_staging(es_plan* p) {
   return ES_OK;
 }
 
-// forward transform of a real box into the X (into_T = false) or T spectrum; rows -> y -> z
-int forward_into(es_plan* p, const float* in, float scale, bool into_T, cudaStream_t s) {
-  float2* mainp = into_T ? p->T : p->X;
-  float2* nyq = into_T ? p->Tnyq : p->Xnyq;
-  const int spec = into_T ? SPEC_T : SPEC_X;
+// the spectrum that the plain transforms use (the first one of a plan for transforms alone)
+int fft_spec(const es_plan* p) { return p->fft_only ? 0 : SPEC_T; }
+
+// forward transform of a real box into spectrum `spec`; rows -> y -> z
+int forward_into(es_plan* p, const float* in, float scale, int spec, cudaStream_t s) {
+  float2* mainp = p->spec[spec];
+  float2* nyq = p->spec_nyq[spec];
   const bool cw = uses_col_warp(p, false);
   es::OpArgs a = base_args(p);
   a.rin = reinterpret_cast<const float2*>(in);
@@ -651,7 +654,54 @@ int forward_into(es_plan* p, const float* in, float scale, bool into_T, cudaStre
   return run_op(p, es::OP_COL_Z_FWD, a, grid_col_z(p, false), s);
 }
 
+// inverse transform of spectrum `spec` (overwritten) into a real box times scale; z -> y -> rows
+int inverse_from(es_plan* p, int spec, float scale, float* out, cudaStream_t s) {
+  es::OpArgs a = base_args(p);
+  a.cin = p->spec[spec]; a.cin_nyq = p->spec_nyq[spec]; a.cout = p->spec[spec]; a.cout_nyq = p->spec_nyq[spec];
+  set_maps(a, p, spec, spec, true, uses_col_warp(p, false));
+  if (int rc = run_op(p, es::OP_COL_Z_INV, a, grid_col_z(p, false), s)) return rc;
+  a = base_args(p);
+  a.cin = p->spec[spec]; a.cin_nyq = p->spec_nyq[spec]; a.cout = p->spec[spec];
+  set_maps(a, p, spec, spec, false, uses_col_warp(p, true));
+  if (int rc = run_op(p, es::OP_COL_Y_INV, a, grid_col_y(p), s)) return rc;
+  a = base_args(p);
+  a.cin = p->spec[spec];
+  a.rout = reinterpret_cast<float2*>(out);
+  a.scale = scale;
+  return run_op(p, es::OP_ROW_C2R_STORE, a, grid_row(p), s);
+}
+
+// SM count and L2 size of the plan's device
+int device_facts(es_plan* p) {
+  int l2 = 0;
+  if (cudaDeviceGetAttribute(&p->sms, cudaDevAttrMultiProcessorCount, p->device) != cudaSuccess ||
+      cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, p->device) != cudaSuccess)
+    return fail(ES_E_CUDA, "cudaDeviceGetAttribute failed");
+  p->l2_bytes = l2;
+  return ES_OK;
+}
+
+// workspace of a plan for transforms alone
+struct FftLayout { size_t main[kMaxSpectra], nyq[kMaxSpectra], counters, total; };
+FftLayout fft_layout(int n, int spectra) {
+  const size_t N = n, M = n / 2;
+  FftLayout L{};
+  size_t off = 0;
+  auto take = [&](size_t bytes) { size_t o = off; off = align_up(off + bytes, 256); return o; };
+  for (int i = 0; i < spectra; ++i) {
+    L.main[i] = take(N * N * M * 8);
+    L.nyq[i] = take(N * N * 8);
+  }
+  L.counters = take(256);
+  L.total = off;
+  return L;
+}
+
 }  // namespace
+
+// ic.cu: folds the shaped half spectrum of an n^3 field onto h^3 (see ic_sampled_fields)
+__attribute__((visibility("hidden"))) cudaError_t ic_launch_fold(int n, int h, float dk, const float2* half, const float2* nyq, int filter, float R, int ref_compat,
+                           int first, int count, float2* const* out, float2* const* out_nyq, cudaStream_t s);
 
 extern "C" {
 
@@ -697,10 +747,7 @@ int es_plan_create(int n, double box_len, int max_radii, es_plan** out) {
   se->geom(&p->geo);
   auto cleanup = [&](int code) { es_plan_destroy(p); return code; };
   if (cudaGetDevice(&p->device) != cudaSuccess) return cleanup(fail(ES_E_CUDA, "no CUDA device"));
-  cudaDeviceProp prop;
-  if (cudaGetDeviceProperties(&prop, p->device) != cudaSuccess) return cleanup(fail(ES_E_CUDA, "cudaGetDeviceProperties failed"));
-  p->sms = prop.multiProcessorCount;
-  p->l2_bytes = prop.l2CacheSize;
+  if (int rc = device_facts(p)) return cleanup(rc);
   p->partial_floats = partial_floats_for(p->sms, p->geo);
   Layout L = layout(n, max_radii, p->partial_floats);
   if (cudaMalloc(&p->base, L.total) != cudaSuccess) {
@@ -712,6 +759,8 @@ int es_plan_create(int n, double box_len, int max_radii, es_plan** out) {
   p->X = (float2*)(b + L.X); p->Xnyq = (float2*)(b + L.Xnyq);
   p->T = (float2*)(b + L.T); p->Tnyq = (float2*)(b + L.Tnyq);
   p->T2 = (float2*)(b + L.T2); p->Tnyq2 = (float2*)(b + L.Tnyq2);
+  p->spec[SPEC_X] = p->X; p->spec[SPEC_T] = p->T; p->spec[SPEC_T2] = p->T2;
+  p->spec_nyq[SPEC_X] = p->Xnyq; p->spec_nyq[SPEC_T] = p->Tnyq; p->spec_nyq[SPEC_T2] = p->Tnyq2;
   p->tw = (float2*)(b + L.tw);
   p->dR[0] = (float*)(b + L.dR0); p->dR[1] = (float*)(b + L.dR1);
   p->flags = (uint32_t*)(b + L.flags);
@@ -771,12 +820,14 @@ int es_plan_destroy(es_plan* p) {
 
 int es_forward(es_plan* p, const float* delta, void* stream) {
   if (!p || !delta) return fail(ES_E_ARG, "es_forward: NULL argument");
+  if (p->fft_only) return fail(ES_E_UNSUPPORTED, "es_forward: the plan is for transforms alone");
   DeviceGuard g(p->device);
-  return forward_into(p, delta, 1.0f, false, (cudaStream_t)stream);
+  return forward_into(p, delta, 1.0f, SPEC_X, (cudaStream_t)stream);
 }
 
 int es_ionize(es_plan* p, const es_ionize_params* prm, float* out, float* nf, void* stream) {
   if (!p || !prm || !out || !nf) return fail(ES_E_ARG, "es_ionize: NULL argument");
+  if (p->fft_only) return fail(ES_E_UNSUPPORTED, "es_ionize: the plan is for transforms alone");
   const int nr = prm->n_radii;
   if (nr < 1 || nr > p->max_radii || !prm->radii)
     return fail(ES_E_ARG, "es_ionize: n_radii=%d outside [1, %d]", nr, p->max_radii);
@@ -963,6 +1014,7 @@ int es_ionize(es_plan* p, const es_ionize_params* prm, float* out, float* nf, vo
 
 int es_delta_T(es_plan* p, const float* xH, const float* delta, float c, float* dT, float* ave, void* stream) {
   if (!p || !xH || !delta || !dT || !ave) return fail(ES_E_ARG, "es_delta_T: NULL argument");
+  if (p->fft_only) return fail(ES_E_UNSUPPORTED, "es_delta_T: the plan is for transforms alone");
   DeviceGuard g(p->device);
   const size_t N3 = (size_t)p->n * p->n * p->n;
   const int slot = prof_begin(p, ES_PROF_DELTA_T, (cudaStream_t)stream);
@@ -978,6 +1030,7 @@ int es_delta_T(es_plan* p, const float* xH, const float* delta, float c, float* 
 int es_power_spectrum(es_plan* p, const float* dT, const float* ave, const int* thr, int nbins,
                       int dimensional, float* out, void* stream) {
   if (!p || !dT || !ave || !thr || !out) return fail(ES_E_ARG, "es_power_spectrum: NULL argument");
+  if (p->fft_only) return fail(ES_E_UNSUPPORTED, "es_power_spectrum: the plan is for transforms alone");
   if (nbins < 1 || nbins > es::PK_MAX_BINS) return fail(ES_E_ARG, "es_power_spectrum: nbins=%d outside [1, %d]", nbins, es::PK_MAX_BINS);
   for (int b = 1; b < nbins; ++b)
     if (thr[b] < thr[b - 1]) return fail(ES_E_ARG, "es_power_spectrum: k^2 thresholds must be non-decreasing");
@@ -1012,32 +1065,89 @@ int es_fft_r2c(es_plan* p, const float* in, void* out, void* stream) {
   if (!p || !in || !out) return fail(ES_E_ARG, "es_fft_r2c: NULL argument");
   DeviceGuard g(p->device);
   cudaStream_t s = (cudaStream_t)stream;
-  int rc = forward_into(p, in, 1.0f, true, s);
+  const int f = fft_spec(p);
+  int rc = forward_into(p, in, 1.0f, f, s);
   if (rc) return rc;
-  to_std_kernel<<<p->sms * 8, 256, 0, s>>>(p->T, p->Tnyq, (float2*)out, p->n);
+  to_std_kernel<<<p->sms * 8, 256, 0, s>>>(p->spec[f], p->spec_nyq[f], (float2*)out, p->n);
   ES_CUDA(cudaGetLastError());
   return ES_OK;
 }
 
-int es_fft_c2r(es_plan* p, const void* in, float* out, void* stream) {
+int es_fft_c2r(es_plan* p, const void* in, float* out, void* stream) { return es_fft_c2r_scaled(p, in, 1.0f, out, stream); }
+
+int es_fft_c2r_scaled(es_plan* p, const void* in, float scale, float* out, void* stream) {
   if (!p || !in || !out) return fail(ES_E_ARG, "es_fft_c2r: NULL argument");
   DeviceGuard g(p->device);
   cudaStream_t s = (cudaStream_t)stream;
-  from_std_kernel<<<p->sms * 8, 256, 0, s>>>((const float2*)in, p->T, p->Tnyq, p->n);
+  const int f = fft_spec(p);
+  from_std_kernel<<<p->sms * 8, 256, 0, s>>>((const float2*)in, p->spec[f], p->spec_nyq[f], p->n);
   ES_CUDA(cudaGetLastError());
-  es::OpArgs a = base_args(p);
-  a.cin = p->T; a.cin_nyq = p->Tnyq; a.cout = p->T; a.cout_nyq = p->Tnyq;
-  set_maps(a, p, SPEC_T, SPEC_T, true, uses_col_warp(p, false));
-  int rc = run_op(p, es::OP_COL_Z_INV, a, grid_col_z(p, false), s);
-  if (rc) return rc;
-  a = base_args(p);
-  a.cin = p->T; a.cin_nyq = p->Tnyq; a.cout = p->T;
-  set_maps(a, p, SPEC_T, SPEC_T, false, uses_col_warp(p, true));
-  if ((rc = run_op(p, es::OP_COL_Y_INV, a, grid_col_y(p), s))) return rc;
-  a = base_args(p);
-  a.cin = p->T;
-  a.rout = reinterpret_cast<float2*>(out);
-  return run_op(p, es::OP_ROW_C2R_STORE, a, grid_row(p), s);
+  return inverse_from(p, f, scale, out, s);
+}
+
+int es_fft_forward(es_plan* p, const float* in, void* stream) {
+  if (!p || !in) return fail(ES_E_ARG, "es_fft_forward: NULL argument");
+  DeviceGuard g(p->device);
+  return forward_into(p, in, 1.0f, fft_spec(p), (cudaStream_t)stream);
+}
+
+size_t es_fft_plan_bytes(int n, int spectra) {
+  if (!find_size(n) || spectra < 1 || spectra > kMaxSpectra) return 0;
+  return fft_layout(n, spectra).total;
+}
+
+int es_fft_plan_create(int n, double box_len, int spectra, const void* twiddles, void* workspace, size_t bytes,
+                       void* stream, es_plan** out) {
+  if (!out) return fail(ES_E_ARG, "es_fft_plan_create: plan pointer is NULL");
+  *out = nullptr;
+  const SizeEntry* se = find_size(n);
+  if (!se) return fail(ES_E_UNSUPPORTED, "es_fft_plan_create: HII_DIM=%d has no compiled kernels", n);
+  if (!(box_len > 0)) return fail(ES_E_ARG, "es_fft_plan_create: BOX_LEN must be positive");
+  if (spectra < 1 || spectra > kMaxSpectra) return fail(ES_E_ARG, "es_fft_plan_create: 1 to %d spectra", (int)kMaxSpectra);
+  const FftLayout L = fft_layout(n, spectra);
+  if (!twiddles || !workspace || ((uintptr_t)workspace & 255) || bytes < L.total)
+    return fail(ES_E_ARG, "es_fft_plan_create: needs a table and %zu bytes of 256-byte aligned workspace", L.total);
+  es_plan* p = new es_plan();
+  p->n = n; p->m = n / 2; p->box_len = box_len; p->size = se; p->fft_only = true; p->nspec = spectra;
+  p->dk = (float)(2.0 * M_PI / (double)(float)box_len);
+  se->geom(&p->geo);
+  auto cleanup = [&](int code) { es_plan_destroy(p); return code; };
+  if (cudaGetDevice(&p->device) != cudaSuccess) return cleanup(fail(ES_E_CUDA, "no CUDA device"));
+  if (int rc = device_facts(p)) return cleanup(rc);
+  char* b = static_cast<char*>(workspace);
+  for (int i = 0; i < spectra; ++i) {
+    p->spec[i] = (float2*)(b + L.main[i]);
+    p->spec_nyq[i] = (float2*)(b + L.nyq[i]);
+  }
+  p->counters = (unsigned*)(b + L.counters);
+  p->err = p->counters + 2;
+  p->tw = (float2*)twiddles;
+  if (int rc = encode_maps(p)) return cleanup(rc);
+  if (int rc = encode_warp_maps(p)) return cleanup(rc);
+  if (cudaMemsetAsync(p->counters, 0, 256, (cudaStream_t)stream) != cudaSuccess)
+    return cleanup(fail(ES_E_CUDA, "es_fft_plan_create: memset failed"));
+  *out = p;
+  return ES_OK;
+}
+
+int ic_sampled_fields(es_plan* big, const void* half, es_plan* small, int filter_type, float R, int ref_compat, int first,
+                      int count, float scale, float* const* out, void* stream) {
+  if (!big || !small || !out) return fail(ES_E_ARG, "ic_sampled_fields: NULL argument");
+  if (filter_type < -1 || filter_type > 2 || first < -1 || count < 1 || first + count > 3 || !small->fft_only ||
+      count > small->nspec || big->device != small->device || big->n % small->n)
+    return fail(ES_E_ARG, "ic_sampled_fields: bad arguments");
+  for (int i = 0; i < count; ++i)
+    if (!out[i]) return fail(ES_E_ARG, "ic_sampled_fields: NULL output");
+  DeviceGuard g(big->device);
+  cudaStream_t s = (cudaStream_t)stream;
+  const int f = fft_spec(big);
+  const float2* src = half ? (const float2*)half : big->spec[f];
+  const cudaError_t e = ic_launch_fold(big->n, small->n, big->dk, src, half ? nullptr : big->spec_nyq[f], filter_type, R,
+                                       ref_compat, first, count, small->spec, small->spec_nyq, s);
+  if (e != cudaSuccess) return fail(ES_E_CUDA, "ic_sampled_fields: launch failed: %s", cudaGetErrorString(e));
+  for (int i = 0; i < count; ++i)
+    if (int rc = inverse_from(small, i, scale, out[i], s)) return rc;
+  return ES_OK;
 }
 
 // ------------------------------------------------------------------ allocation-free delta_T
@@ -1180,6 +1290,7 @@ int es_plan_check(es_plan* p, void* stream) {
 
 int es_profile_enable(es_plan* p, int max_launches) {
   if (!p || max_launches < 0 || max_launches > (1 << 22)) return fail(ES_E_ARG, "es_profile_enable: bad arguments");
+  if (p->fft_only) return fail(ES_E_UNSUPPORTED, "es_profile_enable: the plan is for transforms alone");
   DeviceGuard g(p->device);
   ES_CUDA(cudaDeviceSynchronize());
   for (cudaEvent_t e : p->prof_events) cudaEventDestroy(e);

@@ -798,7 +798,7 @@ __global__ void __launch_bounds__(RowCfg<N>::T) row_c2r(OpArgs a) {
     __syncthreads();
     float2* Zr = fft_lines<M, true, RL, T, false, 1, M, N>(A, B, tw);
     if (EPI == EPI_STORE) {
-      for (int e = threadIdx.x; e < RL * M; e += T) a.rout[base + e] = Zr[e];
+      for (int e = threadIdx.x; e < RL * M; e += T) a.rout[base + e] = cscale(Zr[e], a.scale);
     } else {
       for (int e = threadIdx.x; e < RL * M; e += T) {   // whole warps: 64 consecutive voxels
         const float2 d = Zr[e];

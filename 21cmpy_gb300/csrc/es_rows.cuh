@@ -221,7 +221,7 @@ __global__ void __launch_bounds__(RowTile<N, V>::T, RowOcc<N, V>::MINB) row2_c2r
       if (EPI == EPI_STORE) {
         last_stage_to_regs<M, true, RL, T, ES, N, RS>(Y, tw, [&](int l, int j, const float2* v) {
 #pragma unroll
-          for (int r = 0; r < RLAST; ++r) a.rout[pair0 + (size_t)l * M + j + r * NSL] = v[r];
+          for (int r = 0; r < RLAST; ++r) a.rout[pair0 + (size_t)l * M + j + r * NSL] = cscale(v[r], a.scale);
         });
       } else {
         // one instantiation per (previous radius present, update mode): tests that are uniform
@@ -323,7 +323,7 @@ __global__ void __launch_bounds__(RowTile<N, V>::T, RowOcc<N, V>::MINB) row2_c2r
       if (EPI == EPI_STORE) {
         for (int e = threadIdx.x; e < RL * M; e += T) {
           const int row = e / M, p = e % M;
-          a.rout[pair0 + e] = Zr[p * ES + row];
+          a.rout[pair0 + e] = cscale(Zr[p * ES + row], a.scale);
         }
       } else {
         // one loop per (previous radius present, update mode): tests that are uniform over the

@@ -233,7 +233,7 @@ __global__ void __launch_bounds__(RowWCfg<N>::T, RowOcc<N, 0>::MINB) row_warp_c2
     float2* out = a.rout + row0 + j;
     if (EPI == EPI_STORE) {
 #pragma unroll
-      for (int r = 0; r < R1; ++r) out[r * NSL] = z[r];
+      for (int r = 0; r < R1; ++r) out[r * NSL] = cscale(z[r], a.scale);
       continue;
     }
     // the erfc sum first: the chains are independent and overlap

@@ -14,6 +14,7 @@ All of them run on the CUDA engine; there is no CPU path.
 from __future__ import annotations
 
 import ctypes as C
+import threading
 
 import numpy as np
 import torch
@@ -222,3 +223,106 @@ class ExcursionSetPlan:
 
     def __exit__(self, *exc):
         self.close()
+
+
+_twiddle_tables: dict = {}
+_twiddle_lock = threading.Lock()
+
+
+def _twiddles(n: int, device) -> torch.Tensor:
+    """exp(-2 pi i m / n), m < n, complex64 on the device: a constant per size and device, kept."""
+    key = (n, str(device))
+    with _twiddle_lock:
+        if key not in _twiddle_tables:
+            t = np.exp(-2j * np.pi * np.arange(n) / n).astype(np.complex64)
+            _twiddle_tables[key] = torch.from_numpy(t).to(device)       # from pageable memory: done on return
+        return _twiddle_tables[key]
+
+
+class FftPlan(ExcursionSetPlan):
+    """The engine's real transforms alone (``fft_r2c``, ``fft_c2r``, ``forward_spectrum``), in a workspace
+    from torch's allocator with room for ``spectra`` spectra: cheap to create and to drop.
+
+    Like any tensor, it belongs to the stream that is current where it is made; other streams are to
+    be ordered after that one before they use it."""
+
+    def __init__(self, n: int, box_len: float, spectra: int = 1, device=None):
+        if not torch.cuda.is_available():
+            raise _lib.EngineUnavailable("the excursion-set engine needs a CUDA device")
+        self.lib = _lib.load()
+        self._h = None
+        self.device = torch.device(device) if device is not None else torch.device("cuda", torch.cuda.current_device())
+        if self.device.type != "cuda":
+            raise ValueError("plans live on a CUDA device")
+        if self.device.index is None:
+            self.device = torch.device("cuda", torch.cuda.current_device())
+        self.n, self.box_len, self.max_radii, self.spectra = int(n), float(box_len), 0, int(spectra)
+        nbytes = int(self.lib.es_fft_plan_bytes(self.n, self.spectra))
+        handle = C.c_void_p()
+        with torch.cuda.device(self.device):
+            if nbytes:
+                self._ws = torch.empty(nbytes, dtype=torch.uint8, device=self.device)
+                self._tw = _twiddles(self.n, self.device)
+            rc = self.lib.es_fft_plan_create(self.n, self.box_len, self.spectra, _ptr(self._tw) if nbytes else None,
+                                             _ptr(self._ws) if nbytes else None, nbytes,
+                                             _stream_handle(self.device, None), C.byref(handle))
+        _lib.check("es_fft_plan_create", rc, self.lib)
+        self._h = handle
+
+    def workspace_bytes(self) -> int:
+        return int(self.lib.es_fft_plan_bytes(self.n, self.spectra))
+
+    def _on(self, stream):
+        """The stream's handle; the workspace is not given to others before its work there is done."""
+        s = stream if stream is not None else torch.cuda.current_stream(self.device)
+        self._ws.record_stream(s)
+        return C.c_void_p(s.cuda_stream)
+
+    def forward_spectrum(self, x: torch.Tensor, stream=None):
+        """Unnormalised forward transform into the plan's own spectrum (for ``sampled_fields``)."""
+        self._check_box(x, "x")
+        _lib.check("es_fft_forward", self.lib.es_fft_forward(self.handle, _ptr(x), self._on(stream)), self.lib)
+
+    def fft_r2c(self, x: torch.Tensor, stream=None) -> torch.Tensor:
+        self._on(stream)
+        return super().fft_r2c(x, stream)
+
+    def fft_c2r(self, X: torch.Tensor, stream=None, scale: float = 1.0) -> torch.Tensor:
+        """Unnormalised inverse times ``scale`` from numpy's rfftn layout."""
+        n = self.n
+        if X.dtype != torch.complex64 or tuple(X.shape) != (n, n, n // 2 + 1) or X.device != self.device:
+            raise ValueError("X must be a complex64 (n, n, n/2+1) device tensor")
+        X = X.contiguous()
+        out = torch.empty((n, n, n), dtype=torch.float32, device=self.device)
+        rc = self.lib.es_fft_c2r_scaled(self.handle, _ptr(X), C.c_float(float(np.float32(scale))), _ptr(out), self._on(stream))
+        _lib.check("es_fft_c2r_scaled", rc, self.lib)
+        return out
+
+    def close(self):
+        super().close()
+        self._ws = None
+
+
+def can_sample(dim: int, hii_dim: int, pixel_factor) -> bool:
+    """Whether the HII_DIM^3 nearest cells at this pixel factor are every p-th cell (p whole) and the
+    engine has transforms of both sizes, so that ``sampled_fields`` applies."""
+    return dim % hii_dim == 0 and float(np.float32(pixel_factor)) == dim // hii_dim and \
+        {int(dim), int(hii_dim)} <= set(supported_sizes())
+
+
+def sampled_fields(big: ExcursionSetPlan, half, small: FftPlan, first: int, count: int, R: float, scale: float,
+                   filter_type: int = 0, ref_compat: bool = False) -> list:
+    """Every p-th cell of the smoothed density (component -1) and displacement components (0..2) of a
+    half spectrum (numpy layout; None: the spectrum ``big`` holds), on the current stream."""
+    if half is not None:
+        n = big.n
+        if half.dtype != torch.complex64 or tuple(half.shape) != (n, n, n // 2 + 1) or half.device != big.device \
+                or not half.is_contiguous():
+            raise ValueError("half must be a contiguous complex64 (n, n, n/2+1) device tensor")
+    outs = [torch.empty((small.n,) * 3, dtype=torch.float32, device=small.device) for _ in range(count)]
+    ptrs = (C.c_void_p * count)(*[o.data_ptr() for o in outs])
+    rc = small.lib.ic_sampled_fields(big.handle, None if half is None else _ptr(half), small.handle, int(filter_type),
+                                     C.c_float(float(R)), int(ref_compat), int(first), int(count),
+                                     C.c_float(float(np.float32(scale))), ptrs, small._on(None))
+    _lib.check("ic_sampled_fields", rc, small.lib)
+    return outs

@@ -3,10 +3,11 @@ subsampled copy, and the Zel'dovich displacement (velocity / D-dot) boxes that p
 the mass with (21cmpy's Programs/initialize.py:33-111, initialize.cu:58-95, 133-190).
 
 Pipeline per box: normals -> ``ic_spectrum`` (sqrt(P V) per mode, P linearly interpolated in a
-512-entry table as the reference does) -> the engine's inverse real FFT (``es_fft_c2r``) -> scale;
-for the smoothed density and each displacement component, ``ic_shape`` (window W(kR) with
-R = L_FACTOR * BOX_LEN / HII_DIM, times i k_c / k^2) -> inverse FFT -> ``ic_subsample`` (nearest
-cell, scaled).  Normals come from a seeded torch generator on the device (the reference uses
+512-entry table as the reference does) -> the engine's inverse real FFT and scale
+(``es_fft_c2r_scaled``); for the smoothed density and the displacement components, the window W(kR)
+with R = L_FACTOR * BOX_LEN / HII_DIM and i k_c / k^2, of which every (DIM / HII_DIM)-th cell is kept:
+the shaped spectrum folded onto HII_DIM^3 and transformed there (``ic_sampled_fields``), or, where
+DIM / HII_DIM is not whole, ``ic_shape`` -> inverse FFT -> ``ic_subsample`` (nearest cell) one by one.  Normals come from a seeded torch generator on the device (the reference uses
 PyCUDA's MRG32k3a); they can also be passed in.
 """
 from __future__ import annotations
@@ -40,14 +41,18 @@ class InitialConditions:
     """Initial-conditions boxes for a DIM^3 field of side box_len and its HII_DIM^3 copies."""
 
     def __init__(self, dim: int, hii_dim: int, box_len: float, cosmo=cosmology.PLANCK13, device=None):
-        from .engine import ExcursionSetPlan
+        from .engine import FftPlan, can_sample
         self.lib = _lib.load()
         self.device = torch.device(device) if device is not None else torch.device("cuda", torch.cuda.current_device())
         if self.device.index is None:
             self.device = torch.device("cuda", torch.cuda.current_device())
         self.dim, self.hii_dim, self.box_len = int(dim), int(hii_dim), float(np.float32(box_len))
         self.cosmo = cosmo
-        self.plan = ExcursionSetPlan(self.dim, self.box_len, max_radii=1, device=self.device)
+        self._plan = None
+        self._fft = FftPlan(self.dim, self.box_len, device=self.device)
+        self._small = None
+        if can_sample(self.dim, self.hii_dim, np.float32(self.dim) / np.float32(self.hii_dim)):
+            self._small = FftPlan(self.hii_dim, self.box_len, spectra=4, device=self.device)
         K, P = pk_table(self.dim, self.box_len, cosmo)
         self.K = torch.from_numpy(K).to(self.device)
         self.P = torch.from_numpy(P).to(self.device)
@@ -55,6 +60,15 @@ class InitialConditions:
         self.smooth_R = float(np.float32(L_FACTOR * np.float32(self.box_len) / np.float32(self.hii_dim)))
         # the unnormalised inverse FFT divided by the reference's IFFT normalisation and scale^3
         self.norm = float(1.0 / float(self.box_len) ** 3)
+        torch.cuda.current_stream(self.device).synchronize()     # ready for any stream
+
+    @property
+    def plan(self):
+        """A full plan of DIM^3 boxes, made at first use (the boxes here need transforms alone)."""
+        from .engine import ExcursionSetPlan
+        if self._plan is None:
+            self._plan = ExcursionSetPlan(self.dim, self.box_len, max_radii=1, device=self.device)
+        return self._plan
 
     def _stream(self):
         return C.c_void_p(torch.cuda.current_stream(self.device).cuda_stream)
@@ -95,31 +109,43 @@ class InitialConditions:
         nre, nim = self.normals(seed) if normals is None else normals
         H = self.spectrum(nre, nim)
         out = {"spectrum": H}
-        full = self.plan.fft_c2r(H)
-        out["deltax"] = self.subsample(full, self.norm, size=self.dim, pixel_factor=1.0)
-        del full
-        S = self.plan.fft_c2r(self.shaped(H, -1, filter_type, ref_compat))
+        out["deltax"] = self._fft.fft_c2r(H, scale=self.norm)
+        names = ("smoothed", "vx", "vy", "vz")
+        if self._small is not None:
+            out.update(zip(names, self._sampled(H, -1, 4, self.norm, filter_type, ref_compat)))
+            return out
+        S = self._fft.fft_c2r(self.shaped(H, -1, filter_type, ref_compat))
         out["smoothed"] = self.subsample(S, self.norm)
         del S
         out.update(self.velocities(H, self.norm, filter_type, ref_compat))
         return out
+
+    def _sampled(self, H, first, count, scale, filter_type, ref_compat):
+        from .engine import sampled_fields
+        return sampled_fields(self._fft, H, self._small, first, count, self.smooth_R, scale, filter_type, ref_compat)
 
     def velocities(self, H: torch.Tensor, scale: float, filter_type: int = 0, ref_compat: bool = False,
                    pixel_factor=None) -> dict:
         """{"vx", "vy", "vz"}: scale * IFFT(W(kR) i k_c / k^2 H) subsampled onto HII_DIM^3, the
         inverse FFT unnormalised (set_velocity, HII_filter and subsample: initialize.cu:12-40,
         133-190; perturb_field.cu:39-88)."""
+        from .engine import can_sample
         out = {}
+        pf = self.pixel_factor if pixel_factor is None else pixel_factor
+        if self._small is not None and can_sample(self.dim, self.hii_dim, pf):
+            out.update(zip(("vx", "vy", "vz"), self._sampled(H.contiguous(), 0, 3, scale, filter_type, ref_compat)))
+            return out
         for c, name in enumerate(("vx", "vy", "vz")):
-            V = self.plan.fft_c2r(self.shaped(H, c, filter_type, ref_compat))
+            V = self._fft.fft_c2r(self.shaped(H, c, filter_type, ref_compat))
             out[name] = self.subsample(V, scale, pixel_factor=pixel_factor)
             del V
         return out
 
     def close(self):
-        if getattr(self, "plan", None) is not None:
-            self.plan.close()
-            self.plan = None
+        for p in (self._plan, self._fft, self._small):
+            if p is not None:
+                p.close()
+        self._plan = self._fft = self._small = None
 
     def __enter__(self):
         return self

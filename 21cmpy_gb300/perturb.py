@@ -103,10 +103,23 @@ def updated_velocities(deltax: torch.Tensor, hii_dim: int, box_len: float, growt
     """Velocity boxes of the DIM^3 density ``deltax`` (perturb_field.py:110-125): per component c,
     (dD/dt / D) IFFT(W(kR) i k_c / k^2 FFT(deltax)) with a normalised inverse, R = L_FACTOR *
     BOX_LEN / HII_DIM, subsampled onto HII_DIM^3 (nearest cell).  Returns {"vx", "vy", "vz"}."""
-    from .initial import InitialConditions
+    from .engine import FftPlan, can_sample, sampled_fields
+    from .initial import L_FACTOR, InitialConditions
     dim = int(deltax.shape[0])
     _check_f32(deltax, (dim,) * 3, "deltax", deltax.device)
+    scale = float(np.float32(growth_rate)) / float(dim) ** 3
+    hii, pf = int(hii_dim), np.float32(dim) / np.float32(hii_dim) if pixel_factor is None else pixel_factor
+    if can_sample(dim, hii, pf):
+        # transforms only, in memory from the allocator: the spectrum is folded where the forward
+        # transform leaves it
+        L = float(np.float32(box_len))
+        R = float(np.float32(L_FACTOR * np.float32(L) / np.float32(hii)))
+        with torch.cuda.device(deltax.device):
+            big, small = FftPlan(dim, L, device=deltax.device), FftPlan(hii, L, spectra=3, device=deltax.device)
+            with big, small:
+                big.forward_spectrum(deltax)
+                v = sampled_fields(big, None, small, 0, 3, R, scale, filter_type, ref_compat)
+        return dict(zip(("vx", "vy", "vz"), v))
     with InitialConditions(dim, hii_dim, box_len, device=deltax.device) as ic:
-        H = ic.plan.fft_r2c(deltax)
-        scale = float(np.float32(growth_rate)) / float(dim) ** 3
+        H = ic._fft.fft_r2c(deltax)
         return ic.velocities(H, scale, filter_type, ref_compat, pixel_factor=pixel_factor)

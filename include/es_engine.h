@@ -154,6 +154,21 @@ int es_power_spectrum(es_plan* plan, const float* dT, const float* ave, const in
 int es_fft_r2c(es_plan* plan, const float* in, void* out_half, void* stream);
 int es_fft_c2r(es_plan* plan, const void* in_half, float* out, void* stream);
 
+/* The same inverse with every output times scale (one rounding more, as a separate multiplication). */
+int es_fft_c2r_scaled(es_plan* plan, const void* in_half, float scale, float* out, void* stream);
+
+/* A plan for transforms alone, on a workspace the caller owns (device memory, 256-byte aligned,
+ * es_fft_plan_bytes(n, spectra) bytes; it must outlive the plan) with `spectra` (1..4) spectra in it,
+ * and the table twiddles[m] = exp(-2 pi i m / n), m < n (device complex64).  Creating it launches one
+ * memset on the stream and allocates nothing on the device.  It serves es_fft_r2c, es_fft_c2r(_scaled),
+ * es_fft_forward, ic_sampled_fields, the options, es_plan_check and es_plan_destroy; es_forward,
+ * es_ionize, es_delta_T, es_power_spectrum and es_profile_enable return ES_E_UNSUPPORTED. */
+size_t es_fft_plan_bytes(int n, int spectra);
+int es_fft_plan_create(int n, double box_len, int spectra, const void* twiddles, void* workspace, size_t bytes,
+                       void* stream, es_plan** plan);
+/* Forward transform into the plan's own spectrum, for ic_sampled_fields. */
+int es_fft_forward(es_plan* plan, const float* in, void* stream);
+
 /* Per-launch timing.  es_profile_enable(plan, K) pre-creates event pairs for K launches (0
  * turns timing off); every kernel the plan launches afterwards is bracketed by CUDA events on
  * its stream.  es_profile_read synchronises on the recorded events and writes, per kernel kind
@@ -304,6 +319,15 @@ int ic_spectrum(int n, float box_len, const float* normals_re, const float* norm
                 const float* p_table, int table_n, void* out_half, void* stream);
 int ic_shape(int n, float box_len, const void* in_half, int component, int filter_type, float R, int ref_compat,
              void* out_half, void* stream);
+/* The boxes that ic_shape, the inverse transform and ic_subsample make of a DIM^3 field's half spectrum
+ * where every (DIM / HII_DIM)-th cell is kept, for components first .. first + count - 1 (-1: density,
+ * 0..2: i k_c / k^2; set_velocity, HII_filter and subsample, initialize.cu:12-40, 133-190): sampling
+ * every p-th cell is folding the spectrum p-fold onto itself, so the shaped spectrum is folded to
+ * HII_DIM^3 in one reading and only HII_DIM^3 inverse transforms follow.  big: a plan of DIM (its
+ * own spectrum, es_fft_forward, is used when half is NULL); small: an es_fft_plan of HII_DIM with at
+ * least count spectra; DIM must be a multiple of HII_DIM.  out[i]: device float HII_DIM^3, times scale. */
+int ic_sampled_fields(es_plan* big, const void* half, es_plan* small, int filter_type, float R, int ref_compat, int first,
+                      int count, float scale, float* const* out, void* stream);
 int ic_subsample(int dim, int hii_dim, float pixel_factor, float scale, const float* large, float* small,
                  void* stream);
 int ic_last_error(char* buf, int len);
