@@ -17,24 +17,33 @@
 // reading it, and all slots start zeroed.
 //
 // Shared memory holds every weight, per (dz, dx) as [ci / 8][dy, co][ci % 8] (K-major, no swizzle),
-// and a ring of YS input-row groups; a group is the three rows (z - 1, z, z + 1) at one y, each
-// stored per 8-channel chunk as 130 16-byte positions, position p holding voxel x = (p - 1) mod 128,
-// so shift dx reads the 128 rows starting at position 1 + dx: the circular wrap in x costs nothing.
-// A group is used by exactly one round of MMAs and released right after it.  The copies are
-// 16-byte cp.async by four producer warps (each warp reads 512 contiguous bytes per instruction);
-// a producer keeps three groups in flight and publishes a group with a proxy fence and an mbarrier
-// arrive once its own copies have landed.
+// and a ring of YS input-row groups; a group is the three rows (z - 1, z, z + 1) at one y.  A row lies as
+// in memory, one voxel's channels (64 or 32 bytes) after another, swizzled over that span (K-major
+// operand), with the circular neighbours of its ends before and behind it, so that shift dx starts the
+// operand one voxel earlier or later.  A row comes by three TMA copies: its 128 voxels, and the 128 bytes
+// that end (begin) the row once more in front of (behind) it.  A group is used by exactly one round of MMAs
+// and released right after it.
 //
-// Roles: warps 0..3 copy; warp 4 issues the MMAs (one elected lane) and commits completion to mbarriers;
-// warps 5..8 read finished accumulators (tcgen05.ld, one TMEM lane = one voxel per thread), zero
-// them, add the bias and apply ReLU / sigmoid / the input-gradient mask, and store BF16 (or FP32)
-// rows.  Every wait is bounded; on a timeout the CTA records the error, drains its copies and
-// MMAs, frees its TMEM and leaves.
+// What bounds it: the operands' way out of shared memory, 7168 bytes per MMA of N = 96 at 128 bytes a
+// cycle: 56 cycles, 1008 a row, 53 us a launch.  Copied by 16-byte cp.async into a layout of 8-channel
+// chunks, as before, a group took its producers ~2000 cycles (the pieces land one by one, and each group needed
+// a proxy fence): a 32 -> 32 layer 142 us, now 106.  The rest is the MMA
+// warp's own work between rows (waits, commits, descriptors: ~700 cycles of dependent instructions).
+//
+// Roles: warp 0 issues the copies (one lane); warp 1 issues the MMAs (one elected lane) and commits
+// completion to mbarriers; warps 2..9, two groups that take output rows in turn, read finished
+// accumulators (tcgen05.ld, one TMEM lane = one voxel per thread), zero them, add the bias and apply
+// ReLU / sigmoid / the input-gradient mask (read ahead of the accumulator), and store BF16 (or FP32)
+// rows.  Every wait is bounded; on a timeout the CTA records the error, drains its copies and MMAs, frees
+// its TMEM and leaves.
+#include <cuda.h>
+#include <cudaTypedefs.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
 #include <cstdio>
+#include <mutex>
 #include <string>
 #include <type_traits>
 
@@ -43,15 +52,10 @@
 namespace sgtc {
 
 constexpr int N = 128;                 // box side: one x-row is one M = 128 tile
-constexpr int POS = N + 2;             // 16-byte positions per 8-channel chunk of a staged row
-constexpr int XOFF = 1;                // position of x = 0
-constexpr int CHUNK = POS * 16;        // 2080: distance between the K core matrices of A
 constexpr int YS = 6;                  // input-row groups in the ring
-constexpr int INFLIGHT = 3;            // groups a producer thread keeps in flight (<= YS - 2)
-constexpr int PRODUCERS = 128;         // warps 0..3
-constexpr int MMA_WARP = 4;
-constexpr int EPI_GROUPS = 1;          // epilogue warpgroups, taking output rows in turn
-constexpr int THREADS = 32 * (MMA_WARP + 1 + 4 * EPI_GROUPS);   // + warp 4 (MMA) + warps 5..8 (epilogue)
+constexpr int CONV_MMA_WARP = 1;
+constexpr int EPI_GROUPS = 2;          // epilogue warpgroups of the convolutions, taking output rows in turn
+constexpr int CONV_THREADS = 32 * (2 + 4 * EPI_GROUPS);
 constexpr uint32_t TMEM_COLS = 512;
 constexpr long kSpin = 1L << 24;       // mbarrier polls before a wait is declared hung
 constexpr unsigned ERR_TIMEOUT = 1u;
@@ -66,14 +70,20 @@ template <int CIN, int COUT> struct Layout {
   static constexpr int LBO_B = 3 * COUT * 16;         // B: K core matrices 3 * COUT rows apart
   static constexpr int PAIR_B = KC * LBO_B;           // B of one (dz, dx): 3 taps
   static constexpr int W_BYTES = 9 * PAIR_B;
-  static constexpr int ROW_BYTES = KC * CHUNK;
-  static constexpr int RING_BYTES = YS * 3 * ROW_BYTES;
-  static constexpr int BAR_OFF = W_BYTES + RING_BYTES;
+  static constexpr int VOX = CIN * 2;                  // bytes of a voxel: the swizzle span
+  static constexpr int PAD = 512;                      // before and between rows: 128 bytes of either neighbour's ends
+  static constexpr int ROW = N * VOX + PAD;            // from row to row
+  static constexpr int GROUP = 3 * ROW;
+  static constexpr int HALO = 128 / VOX;               // voxels of an end copy (128 bytes)
+  static constexpr uint32_t GROUP_TX = 3 * (N * VOX + 2 * 128);
+  static constexpr int RING_BYTES = PAD + YS * GROUP;
+  static constexpr int W_OFF = (RING_BYTES + 127) / 128 * 128;
+  static constexpr int BAR_OFF = W_OFF + W_BYTES;
   static constexpr int NBARS = 2 * YS + 2 * S + 1;    // full[YS], sfree[YS], done[S], tfree[S], drain
-  static constexpr int BYTES = BAR_OFF + NBARS * 8 + 16 + 128;   // + tmem slot, abort, alignment
-  static_assert(W_BYTES % 16 == 0 && ROW_BYTES % 16 == 0, "16-byte aligned regions");
+  static constexpr int BYTES = BAR_OFF + NBARS * 8 + 16 + 1024;   // + tmem slot, abort, alignment
+  static_assert(VOX == 64 || VOX == 32, "a voxel is one swizzle span");
+  static_assert(W_BYTES % 16 == 0, "16-byte aligned regions");
   static_assert(3 * COUT <= 256 && COUT % 16 == 0, "N = 3 COUT must be a valid M = 128 MMA width");
-  static_assert(INFLIGHT <= YS - 2, "a producer must not wait on a slot its own pending groups hold");
   static_assert(BYTES <= 232448, "shared memory per CTA");
 };
 
@@ -106,15 +116,17 @@ __device__ __forceinline__ bool bar_wait(uint64_t* b, uint32_t parity, volatile 
   atomicOr(&g_err, ERR_TIMEOUT);
   return false;
 }
-__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(saddr(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int K> __device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;" ::"n"(K) : "memory");
-}
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void fence_bar_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
+__device__ __forceinline__ void bar_expect_tx(uint64_t* b, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(saddr(b)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void tma_load3(void* dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1, int c2) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+      ::"r"(saddr(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(saddr(bar))
+      : "memory");
+}
 __device__ __forceinline__ void tc_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
@@ -134,6 +146,12 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t cols) {
 __device__ __forceinline__ uint64_t mdesc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
   return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) |
          ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46);
+}
+// The same, K-major with rows of VOX = 64 or 32 bytes swizzled over that span: 8-row groups one after
+// another; the pattern goes by the address, so a start inside a group needs no more.
+template <int VOX> __device__ __forceinline__ uint64_t mdesc_rows(uint32_t addr) {
+  return (uint64_t)((addr >> 4) & 0x3FFFu) | (1ull << 16) | ((uint64_t)((8 * VOX) >> 4) << 32) | (1ull << 46) |
+         ((VOX == 64 ? 4ull : 6ull) << 61);
 }
 // Instruction descriptor of kind::f16: FP32 accumulator, BF16 A and B, both K-major, M x N.
 __host__ __device__ constexpr uint32_t idesc_bf16(int m, int n) {
@@ -200,18 +218,37 @@ __device__ __forceinline__ Range my_rows() {
   return {(int)((long)rows * blockIdx.x / gridDim.x), (int)((long)rows * (blockIdx.x + 1) / gridDim.x)};
 }
 
+// The input-row groups of a CTA in order: per z-plane segment [yb, ye) of its output rows, y = yb - 1 .. ye.
+struct GroupWalk {
+  int r, r1, z, ye, yy;
+  __device__ __forceinline__ GroupWalk(Range rg) : r(rg.r0), r1(rg.r1) { segment(); }
+  __device__ __forceinline__ void segment() {
+    z = r / N;
+    ye = (z + 1) * N < r1 ? N : r1 - z * N;
+    yy = r % N - 1;
+  }
+  __device__ __forceinline__ bool done() const { return r >= r1; }
+  __device__ __forceinline__ void next() {
+    if (++yy > ye) {
+      r = z * N + ye;
+      segment();
+    }
+  }
+};
+
 template <int CIN, int COUT, int MODE>
-__global__ void __launch_bounds__(THREADS, 1) conv_tc_kernel(const __nv_bfloat16* __restrict__ in,
-                                                             const __nv_bfloat16* __restrict__ w,
-                                                             const float* __restrict__ bias, void* out,
-                                                             const __nv_bfloat16* __restrict__ mask) {
+__global__ void __launch_bounds__(CONV_THREADS, 1) conv_tc_kernel(const __grid_constant__ CUtensorMap tm_row,
+                                                                  const __grid_constant__ CUtensorMap tm_end,
+                                                                  const __nv_bfloat16* __restrict__ w,
+                                                                  const float* __restrict__ bias, void* out,
+                                                                  const __nv_bfloat16* __restrict__ mask) {
   using L = Layout<CIN, COUT>;
   constexpr int KC = L::KC, S = L::S;
   constexpr int KSTEPS = CIN / 16;                    // MMA K steps per (dz, dx)
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
-  unsigned char* sw = sm;
-  unsigned char* ring = sm + L::W_BYTES;
+  unsigned char* sm = smem_raw + ((0u - saddr(smem_raw)) & 1023u);
+  unsigned char* ring = sm + L::PAD;                  // first voxel of the first row
+  unsigned char* sw = sm + L::W_OFF;
   uint64_t* bars = reinterpret_cast<uint64_t*>(sm + L::BAR_OFF);
   uint64_t* full = bars;
   uint64_t* sfree = bars + YS;
@@ -224,7 +261,7 @@ __global__ void __launch_bounds__(THREADS, 1) conv_tc_kernel(const __nv_bfloat16
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int i = 0; i < YS; ++i) {
-      bar_init(&full[i], PRODUCERS);
+      bar_init(&full[i], 1);
       bar_init(&sfree[i], 1);
     }
     for (int i = 0; i < S; ++i) {
@@ -239,19 +276,53 @@ __global__ void __launch_bounds__(THREADS, 1) conv_tc_kernel(const __nv_bfloat16
     tmem_alloc(tmem_slot, TMEM_COLS);
     tmem_relinquish();
   }
-  // weights -> per (dz, dx): [ci / 8][dy, co][ci % 8], 16-byte chunks
-  for (int c = threadIdx.x; c < 27 * COUT * KC; c += THREADS) {
-    const int kc = c % KC, co = (c / KC) % COUT, t = c / (KC * COUT);
-    const int dz = t / 9, dy = (t / 3) % 3, dx = t % 3;
-    const uint4 v = __ldg(reinterpret_cast<const uint4*>(w + ((size_t)(t * COUT + co) * CIN + kc * 8)));
-    *reinterpret_cast<uint4*>(sw + (dz * 3 + dx) * L::PAIR_B + kc * L::LBO_B + (dy * COUT + co) * 16) = v;
+  __syncthreads();
+  const Range rg = my_rows();
+  GroupWalk walk(rg);
+  int issued = 0;                                     // groups whose copies are under way
+  auto issue_group = [&]() {
+    const int slot = issued % YS;
+    bar_expect_tx(&full[slot], L::GROUP_TX);
+    unsigned char* gb = ring + slot * L::GROUP;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const int row = ((walk.z + d + N - 1) % N) * N + (walk.yy + N) % N;
+      unsigned char* dst = gb + d * L::ROW;
+      tma_load3(dst, &tm_row, &full[slot], 0, 0, row);
+      tma_load3(dst - 128, &tm_end, &full[slot], 0, N - L::HALO, row);
+      tma_load3(dst + N * L::VOX, &tm_end, &full[slot], 0, 0, row);
+    }
+    ++issued;
+    walk.next();
+  };
+  // the first groups are on their way while the weights are staged
+  if (threadIdx.x == 0)
+    while (issued < YS && !walk.done()) issue_group();
+  // weights -> per (dz, dx): [ci / 8][dy, co][ci % 8], 16-byte chunks; all loads of a thread in flight at once
+  {
+    constexpr int WCH = 27 * COUT * KC, Q = (WCH + CONV_THREADS - 1) / CONV_THREADS;
+    uint4 v[Q];
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      const int c = threadIdx.x + q * CONV_THREADS;
+      if (c < WCH) v[q] = __ldg(reinterpret_cast<const uint4*>(w) + c);   // [t][co][kc] is w's own order
+    }
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      const int c = threadIdx.x + q * CONV_THREADS;
+      if (c < WCH) {
+        const int kc = c % KC, co = (c / KC) % COUT, t = c / (KC * COUT);
+        const int dz = t / 9, dy = (t / 3) % 3, dx = t % 3;
+        *reinterpret_cast<uint4*>(sw + (dz * 3 + dx) * L::PAIR_B + kc * L::LBO_B + (dy * COUT + co) * 16) = v[q];
+      }
+    }
   }
   fence_proxy_async();                                // generic writes -> tensor-core reads
   tc_before();
   __syncthreads();
   tc_after();
   const uint32_t tmem = *tmem_slot;
-  if (warp > MMA_WARP && warp <= MMA_WARP + 4) {
+  if (warp > CONV_MMA_WARP && warp <= CONV_MMA_WARP + 4) {
     // every accumulator slot starts at zero
     const uint32_t lanes = (uint32_t)(32 * (warp & 3)) << 16;
     for (int c = 0; c < (int)TMEM_COLS; c += 16) tmem_zero16(tmem + lanes + (uint32_t)c);
@@ -260,94 +331,71 @@ __global__ void __launch_bounds__(THREADS, 1) conv_tc_kernel(const __nv_bfloat16
   tc_before();
   __syncthreads();
   tc_after();
-  const Range rg = my_rows();
 
-  if (warp < MMA_WARP) {
+  if (warp == 0) {
     // ------------------------------------------------------------------ copies
-    // Copy j of a row: position p, chunk kc with kc fastest, so a warp reads 8 whole voxels; the
-    // offsets depend only on the thread and j, so they are computed once.
-    constexpr int PER_ROW = KC * POS, JR = (PER_ROW + PRODUCERS - 1) / PRODUCERS;
-    const int pt = threadIdx.x;
-    uint32_t soff[JR], goff[JR];
-#pragma unroll
-    for (int j = 0; j < JR; ++j) {
-      const int c = pt + j * PRODUCERS, p = c / KC, kc = c % KC;
-      soff[j] = (uint32_t)(kc * CHUNK + p * 16);
-      goff[j] = (uint32_t)(((p + N - 1) % N) * CIN + kc * 8);
+    if (lane == 0) {
+      for (; !walk.done(); issue_group())
+        if (issued >= YS && !bar_wait(&sfree[issued % YS], (uint32_t)((issued / YS - 1) & 1), abort)) break;
+      // no copy outlives the CTA: after an abort every group issued lands first (bounded; otherwise the MMA
+      // warp has seen them all)
+      if (*abort)
+        for (int q = issued > YS ? issued - YS : 0; q < issued; ++q)
+          for (long i = 0; i < kSpin && !bar_try(&full[q % YS], (uint32_t)((q / YS) & 1)); ++i) {
+          }
     }
-    int g = 0, published = 0;
-    for (int r = rg.r0; r < rg.r1 && !*abort;) {
-      const int z = r / N, yb = r % N;
-      const int ye = (z + 1) * N < rg.r1 ? N : rg.r1 - z * N;
-      for (int yy = yb - 1; yy <= ye && !*abort; ++yy) {
-        const int slot = g % YS;
-        if (g >= YS && !bar_wait(&sfree[slot], (uint32_t)((g / YS - 1) & 1), abort)) break;
-        const int yw = (yy + N) % N;
-        unsigned char* gb = ring + slot * 3 * L::ROW_BYTES;
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-          const __nv_bfloat16* src = in + (size_t)(((z + d + N - 1) % N) * N + yw) * N * CIN;
-          unsigned char* dst = gb + d * L::ROW_BYTES;
-#pragma unroll
-          for (int j = 0; j < JR; ++j)
-            if (PER_ROW % PRODUCERS == 0 || pt + j * PRODUCERS < PER_ROW) cp_async16(dst + soff[j], src + goff[j]);
-        }
-        cp_async_commit();
-        ++g;
-        if (g - published >= INFLIGHT) {
-          cp_async_wait<INFLIGHT - 1>();             // the oldest pending group has landed
-          fence_proxy_async();
-          bar_arrive(&full[published % YS]);
-          ++published;
-        }
-      }
-      r = z * N + ye;
-    }
-    cp_async_wait<0>();
-    fence_proxy_async();
-    if (!*abort)
-      for (; published < g; ++published) bar_arrive(&full[published % YS]);
-  } else if (warp == MMA_WARP) {
+  } else if (warp == CONV_MMA_WARP) {
     {
       // ---------------------------------------------------------------- MMA issue
       // Descriptors are a base descriptor plus (byte offset >> 4) in the 14-bit address field.
-      const uint64_t a_base = mdesc(saddr(ring), CHUNK, 128);
+      const uint64_t a_base = mdesc_rows<L::VOX>(saddr(ring));
       const uint64_t b_base = mdesc(saddr(sw), L::LBO_B, 128);
       int g = 0, o0 = 0;
       for (int r = rg.r0; r < rg.r1 && !__any_sync(0xFFFFFFFFu, *abort);) {
         const int z = r / N, yb = r % N;
         const int ye = (z + 1) * N < rg.r1 ? N : rg.r1 - z * N;
-        bool ok = true;
+        // Input row Y's group has landed and output row Y + 1's slot is free.  Freed slots are looked for
+        // eight rows at a time (a wait costs ~200 cycles even when there is nothing to wait for): the
+        // epilogue groups take rows in order, so the last row of either group among the eight speaks for all.
+        auto ready = [&](int Y, int gg) {
+          bool k = bar_wait(&full[gg % YS], (uint32_t)((gg / YS) & 1), abort);
+          const int o = o0 + Y + 1 - yb;
+          if (Y + 1 < ye && o >= S && o % 8 == 0) {
+#pragma unroll
+            for (int e = 0; e < EPI_GROUPS; ++e) {
+              const int q = o + 7 - e;
+              k = k && bar_wait(&tfree[(S - 1) - q % S], (uint32_t)((q / S - 1) & 1), abort);
+            }
+          }
+          return (bool)__all_sync(0xFFFFFFFFu, k);
+        };
+        bool ok = ready(yb - 1, g);
         for (int Y = yb - 1; Y <= ye && ok; ++Y, ++g) {
-          ok = __all_sync(0xFFFFFFFFu, bar_wait(&full[g % YS], (uint32_t)((g / YS) & 1), abort));
           // output rows this input row feeds: y in [ylo, yhi], tap dy = Y - y
           const int ylo = Y - 1 > yb ? Y - 1 : yb, yhi = Y + 1 < ye - 1 ? Y + 1 : ye - 1;
           const int ohi = o0 + (yhi - yb);
-          if (ok && yhi == Y + 1 && ohi >= S)          // first touch of row Y + 1's slot
-            ok = __all_sync(0xFFFFFFFFu, bar_wait(&tfree[(S - 1) - ohi % S], (uint32_t)((ohi / S - 1) & 1), abort));
-          if (!ok) break;
           tc_after();
           const int nrows = yhi - ylo + 1;
           const int s0 = (S - 1) - ohi % S;            // slot of row yhi; rows below follow upward
           const int n1 = nrows < S - s0 ? nrows : S - s0, n2 = nrows - n1;
           const uint32_t id1 = idesc_bf16(128, n1 * COUT), id2 = idesc_bf16(128, (n2 > 0 ? n2 : 1) * COUT);
           const uint32_t d1 = tmem + (uint32_t)(s0 * COUT);
-          const uint64_t a_g = a_base + (uint64_t)((g % YS) * (3 * L::ROW_BYTES / 16));
+          const uint64_t a_g = a_base + (uint64_t)((g % YS) * (L::GROUP / 16));
           const uint64_t b_blk = b_base + (uint64_t)((Y - yhi + 1) * COUT);   // first dy block, 16-byte units
 // One straight run of MMAs per case: a test between the MMAs (whether the slot ring wraps)
           // would put a branch around every elected issue and slow the issue to ~90 cycles per MMA;
           // without it the issue keeps pace with the tensor pipe (~56 cycles at N = 96).
-          auto issue = [&](auto two) {
+          auto issue = [&](auto two, auto from, auto to) {
             constexpr bool TWO = decltype(two)::value;
 #pragma unroll
-            for (int dz = 0; dz < 3; ++dz) {
+            for (int dz = decltype(from)::value; dz < decltype(to)::value; ++dz) {
 #pragma unroll
               for (int dx = 0; dx < 3; ++dx) {
-                const uint64_t ad = a_g + (uint64_t)((dz * L::ROW_BYTES + (XOFF + dx - 1) * 16) / 16);
+                const uint64_t ad = a_g + (uint64_t)(int64_t)((dz * L::ROW + (dx - 1) * L::VOX) / 16);
                 const uint64_t bd = b_blk + (uint64_t)((dz * 3 + dx) * L::PAIR_B / 16);
 #pragma unroll
                 for (int k = 0; k < KSTEPS; ++k) {
-                  const uint64_t ak = ad + (uint64_t)(2 * k * CHUNK / 16);
+                  const uint64_t ak = ad + (uint64_t)(2 * k);      // 16 channels: 32 bytes along the voxel
                   const uint64_t bk = bd + (uint64_t)(2 * k * L::LBO_B / 16);
                   mma_acc(d1, ak, bk, id1);
                   if (TWO) mma_acc(tmem, ak, bk + (uint64_t)(n1 * COUT), id2);
@@ -355,12 +403,21 @@ __global__ void __launch_bounds__(THREADS, 1) conv_tc_kernel(const __nv_bfloat16
               }
             }
           };
-          if (n2 > 0) issue(std::true_type{}); else issue(std::false_type{});
+          // The waits for the next row stand between the second and the third dz: the MMAs queued so far run
+          // meanwhile (waits between rows left the tensor pipe idle ~400 cycles a row)
+          typedef std::integral_constant<int, 0> I0;
+          typedef std::integral_constant<int, 2> I2;
+          typedef std::integral_constant<int, 3> I3;
+          if (n2 > 0) issue(std::true_type{}, I0{}, I2{}); else issue(std::false_type{}, I0{}, I2{});
+          const bool next_ok = Y < ye ? ready(Y + 1, g + 1) : true;
+          tc_after();
+          if (n2 > 0) issue(std::true_type{}, I2{}, I3{}); else issue(std::false_type{}, I2{}, I3{});
           mma_commit(&sfree[g % YS]);                 // this input group is not read again
           if (Y - 1 >= yb && Y - 1 < ye) {
             const int od = o0 + (Y - 1 - yb);          // output row Y - 1 has all 27 taps
             mma_commit(&done[(S - 1) - od % S]);
           }
+          ok = next_ok;
         }
         if (!ok) break;
         o0 += ye - yb;
@@ -380,10 +437,16 @@ __global__ void __launch_bounds__(THREADS, 1) conv_tc_kernel(const __nv_bfloat16
     float bv[COUT];
 #pragma unroll
     for (int c = 0; c < COUT; ++c) bv[c] = bias ? bias[c] : 0.f;
-    const int eg = (warp - MMA_WARP - 1) / 4;         // this warpgroup takes rows o = eg mod EPI_GROUPS
+    const int eg = (warp - CONV_MMA_WARP - 1) / 4;         // this warpgroup takes rows o = eg mod EPI_GROUPS
     for (int o = eg; o < rg.r1 - rg.r0; o += EPI_GROUPS) {
       const int r = rg.r0 + o;
       const int slot = (S - 1) - o % S;
+      const size_t vox = (size_t)r * N + x;
+      uint4 mrow[COUT / 8];                            // the mask's row, on its way while the MMAs finish
+      if (MODE == DGRAD_MASK) {
+#pragma unroll
+        for (int j = 0; j < COUT / 8; ++j) mrow[j] = __ldg(reinterpret_cast<const uint4*>(mask + vox * COUT) + j);
+      }
       const bool ok = bar_wait(&done[slot], (uint32_t)((o / S) & 1), abort);
       if (!__all_sync(0xFFFFFFFFu, ok)) break;        // tcgen05.ld / st need the whole warp
       tc_after();
@@ -395,17 +458,15 @@ __global__ void __launch_bounds__(THREADS, 1) conv_tc_kernel(const __nv_bfloat16
       tmem_wait_st();
       tc_before();
       bar_arrive(&tfree[slot]);
-      const size_t vox = (size_t)r * N + x;
       if (MODE == FWD_SIGMOID) {
         reinterpret_cast<float*>(out)[vox] = 1.0f / (1.0f + __expf(-(v[0] + bv[0])));
       } else {
         uint32_t mbits = 0xFFFFFFFFu;
         if (MODE == DGRAD_MASK) {
-          const uint4* mp = reinterpret_cast<const uint4*>(mask + vox * COUT);
           mbits = 0;
 #pragma unroll
           for (int j = 0; j < COUT / 8; ++j) {
-            const uint4 m = __ldg(mp + j);
+            const uint4 m = mrow[j];
             const uint32_t wds[4] = {m.x, m.y, m.z, m.w};
 #pragma unroll
             for (int h = 0; h < 8; ++h) {
@@ -451,38 +512,45 @@ __global__ void __launch_bounds__(THREADS, 1) conv_tc_kernel(const __nv_bfloat16
 // dW[t][co][ci] = sum_v dZ[v][co] X[v + (dz, dy, dx)][ci] and db[co] = sum_v dZ[v][co] at 128^3.
 // With u = v + (0, 0, dx): dW = sum_u dZ[u - dx][co] X[u + (dz, dy, 0)][ci], so for one output row
 // (z, y) of dZ and one dy, one MMA per 16 voxels covers every (dz, ci) x (dx, co):
-//   A (M = 128, MN-major): the input rows z - 1, z, z + 1 at y + dy with 32 channel slots each, then
-//     a constant row of ones, whose products are the bias gradient;
-//   B (N = 3 COUT, MN-major): the dZ row (z, y) staged three times, shifted by dx = -1, 0, +1 (the
-//     circular wrap in x is applied while staging);
+//   A (M = 128, MN-major): the input rows z - 1, z, z + 1 at y + dy, and a constant row of ones, whose
+//     products are the bias gradient, CIN channels each (with CIN = 16 the upper half of M reads on into
+//     whatever follows and is not used);
+//   B (N = 3 COUT, MN-major): the dZ row (z, y) three times over, starting one voxel early, in place and one
+//     late (dx = +1, 0, -1): with one voxel as the stride between the three, one copy of the row serves;
 //   D: one accumulator per dy (3 COUT columns of tensor memory), summed over all of the CTA's rows.
-// Staged rows hold, per 8-channel chunk, 128 voxel positions of 16 bytes: in MN-major terms the
-// core matrices (8 voxels x 8 channels) are 128 bytes apart along K and one chunk (2048 bytes)
-// apart along M / N, the same stride from a row's last chunk to the next row's first.  For
-// CIN = 16 the chunk slots 2 and 3 of a row are never written; they feed accumulator rows that are
-// not read.  Per-CTA partials [3][128][3 COUT] are summed in a fixed order by wgrad_tc_reduce.
+// Staged rows lie as in memory, swizzled over a voxel's bytes (as in the convolutions), which is the
+// MN-major layout of that swizzle: 8 voxels to a group along K, a row (or a voxel) from one span of
+// channels to the next along M (N).  TMA brings them; a dZ row has its circular neighbours at either
+// end.  Per-CTA partials [3][128][3 COUT] are summed in a fixed order by wgrad_tc_reduce.
+// Bound by the operands' way out of shared memory, 1344 cycles a row, 70 us a launch; with 16-byte cp.async
+// into 8-channel chunks, dZ three times, a 32 x 32 layer took 292 us (the copies, and a proxy fence each);
+// now 112 us.
 namespace wg {
-constexpr int CH = N * 16;                 // 2048 bytes per 8-channel chunk of a staged row
-constexpr int KCS = 4;                     // channel-chunk slots per staged input row
-constexpr int XROW = KCS * CH;             // 8192
-constexpr int XGROUP = 4 * XROW;           // rows z - 1, z, z + 1 and the ones row
-constexpr int XS = 4;                      // input-row groups: y - 1, y, y + 1 in use, y + 2 landing
-constexpr int DSL = 2;                     // dZ row slots
-constexpr int WINFLIGHT = 3;               // items (groups or dZ rows) a producer keeps in flight
+constexpr int XS = 5;                      // input-row groups: y - 1, y, y + 1 in use, two landing
+constexpr int DSL = 4;                     // dZ row slots
+constexpr int PAD = 512;                   // before and between dZ rows: 128 bytes of either neighbour's ends
+constexpr int WG_THREADS = 32 * 6;         // warp 0 copies, warp 1 MMAs, warps 2..5 partials
 }  // namespace wg
 
 template <int CIN, int COUT> struct WLayout {
-  static constexpr int KC = CIN / 8, KCD = COUT / 8;
-  static constexpr int DCOPY = KCD * wg::CH;           // one shifted copy of a dZ row
-  static constexpr int DSLOT = 3 * DCOPY;
+  static constexpr int XV = CIN * 2, DV = COUT * 2;    // bytes of a voxel of X and of dZ: the swizzle spans
+  static constexpr int XROW = N * XV;
+  static constexpr int XGROUP = 4 * XROW;              // rows z - 1, z, z + 1 and the ones row
+  static constexpr int DROW = N * DV + wg::PAD;
+  static constexpr int HALO = 128 / DV;                // voxels of an end copy (128 bytes)
+  static constexpr uint32_t X_TX = 3 * XROW, D_TX = N * DV + 2 * 128;
   static constexpr int NCOLS = 3 * COUT;               // N of one MMA
   static constexpr uint32_t TCOLS = 3 * NCOLS <= 256 ? 256u : 512u;
-  static constexpr int XRING = wg::XS * wg::XGROUP;
-  static constexpr int BAR_OFF = XRING + wg::DSL * DSLOT;
+  static constexpr int ONES = 3 * CIN;                 // accumulator row of the bias gradient
+  static constexpr int XRING = wg::XS * XGROUP;
+  // with CIN = 16 an A operand reads 8 rows' worth from its group: up to a group past the ring
+  static constexpr int D_OFF = XRING + wg::PAD, D_END = D_OFF + wg::DSL * DROW;
+  static constexpr int A_END = XRING + (CIN == 16 ? XGROUP : 0);
+  static constexpr int BAR_OFF = ((D_END > A_END ? D_END : A_END) + 15) / 16 * 16;
   static constexpr int NBARS = 2 * wg::XS + 2 * wg::DSL + 1;    // xfull, xfree, dfull, dfree, done
-  static constexpr int BYTES = BAR_OFF + NBARS * 8 + 16 + 128;
+  static constexpr int BYTES = BAR_OFF + NBARS * 8 + 16 + 1024;
   static_assert(NCOLS % 16 == 0 && NCOLS <= 256, "N = 3 COUT must be a valid M = 128 MMA width");
-  static_assert(KC <= wg::KCS, "at most 32 input channels");
+  static_assert(XGROUP % 512 == 0 && DROW % 512 == 0, "rows start on a whole swizzle pattern");
   static_assert(BYTES <= 232448, "shared memory per CTA");
 };
 
@@ -506,25 +574,26 @@ __device__ __forceinline__ bool wbar_wait(uint64_t* b, uint32_t parity, volatile
   return false;
 }
 
-// Shared-memory matrix descriptor, MN-major without swizzle: core matrices of 8 K-rows x 16 bytes
-// (8 elements along M or N), `lbo` between core matrices along K, `sbo` along M / N.
-__device__ __forceinline__ uint64_t mdesc_mn(uint32_t addr, uint32_t lbo, uint32_t sbo) {
+// Shared-memory matrix descriptor, MN-major with rows of VOX = 64 or 32 bytes (VOX / 2 elements along M or
+// N) swizzled over that span: 8 K-rows to a group, groups one after another, `lbo` from one span along M
+// or N to the next.
+template <int VOX> __device__ __forceinline__ uint64_t mdesc_mn(uint32_t addr, uint32_t lbo) {
   return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) |
-         ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46);
+         ((uint64_t)((8 * VOX) >> 4) << 32) | (1ull << 46) | ((VOX == 64 ? 4ull : 6ull) << 61);
 }
 // kind::f16 instruction descriptor with both operands MN-major (transpose bits 15 and 16)
 __host__ __device__ constexpr uint32_t idesc_bf16_mn(int m, int n) { return idesc_bf16(m, n) | (1u << 15) | (1u << 16); }
 
 template <int CIN, int COUT>
-__global__ void __launch_bounds__(THREADS, 1) wgrad_tc_kernel(const __nv_bfloat16* __restrict__ x,
-                                                              const __nv_bfloat16* __restrict__ dz,
-                                                              float* __restrict__ partials) {
+__global__ void __launch_bounds__(wg::WG_THREADS, 1) wgrad_tc_kernel(const __grid_constant__ CUtensorMap tm_x,
+                                                                     const __grid_constant__ CUtensorMap tm_d,
+                                                                     const __grid_constant__ CUtensorMap tm_dend,
+                                                                     float* __restrict__ partials) {
   using L = WLayout<CIN, COUT>;
-  constexpr int KC = L::KC, KCD = L::KCD;
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
+  unsigned char* sm = smem_raw + ((0u - saddr(smem_raw)) & 1023u);
   unsigned char* xring = sm;
-  unsigned char* dring = sm + L::XRING;
+  unsigned char* dring = sm + L::D_OFF;              // first voxel of the first dZ row
   uint64_t* bars = reinterpret_cast<uint64_t*>(sm + L::BAR_OFF);
   uint64_t* xfull = bars;
   uint64_t* xfree = bars + wg::XS;
@@ -537,11 +606,11 @@ __global__ void __launch_bounds__(THREADS, 1) wgrad_tc_kernel(const __nv_bfloat1
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int i = 0; i < wg::XS; ++i) {
-      bar_init(&xfull[i], PRODUCERS);
+      bar_init(&xfull[i], 1);
       bar_init(&xfree[i], 1);
     }
     for (int i = 0; i < wg::DSL; ++i) {
-      bar_init(&dfull[i], PRODUCERS);
+      bar_init(&dfull[i], 1);
       bar_init(&dfree[i], 1);
     }
     bar_init(done, 1);
@@ -555,9 +624,9 @@ __global__ void __launch_bounds__(THREADS, 1) wgrad_tc_kernel(const __nv_bfloat1
   // the ones row of every input-group slot (bf16 1.0 = 0x3F80), written once
   {
     const uint4 ones = make_uint4(0x3F803F80u, 0x3F803F80u, 0x3F803F80u, 0x3F803F80u);
-    for (int i = threadIdx.x; i < wg::XS * (wg::XROW / 16); i += THREADS) {
-      const int slot = i / (wg::XROW / 16), j = i % (wg::XROW / 16);
-      *reinterpret_cast<uint4*>(xring + slot * wg::XGROUP + 3 * wg::XROW + 16 * j) = ones;
+    for (int i = threadIdx.x; i < wg::XS * (L::XROW / 16); i += wg::WG_THREADS) {
+      const int slot = i / (L::XROW / 16), j = i % (L::XROW / 16);
+      *reinterpret_cast<uint4*>(xring + slot * L::XGROUP + 3 * L::XROW + 16 * j) = ones;
     }
   }
   fence_proxy_async();
@@ -565,7 +634,7 @@ __global__ void __launch_bounds__(THREADS, 1) wgrad_tc_kernel(const __nv_bfloat1
   __syncthreads();
   tc_after();
   const uint32_t tmem = *tmem_slot;
-  if (warp > MMA_WARP && warp <= MMA_WARP + 4) {
+  if (warp > CONV_MMA_WARP) {
     const uint32_t lanes = (uint32_t)(32 * (warp & 3)) << 16;
     for (int c = 0; c < (int)L::TCOLS; c += 16) tmem_zero16(tmem + lanes + (uint32_t)c);
     tmem_wait_st();
@@ -575,89 +644,54 @@ __global__ void __launch_bounds__(THREADS, 1) wgrad_tc_kernel(const __nv_bfloat1
   tc_after();
   const Range rg = my_rows();
 
-  if (warp < MMA_WARP) {
+  if (warp == 0) {
     // ------------------------------------------------------------------ copies
-    // Items in order, per z-plane segment [yb, ye) of the CTA's rows: X(yb - 1), X(yb), then per
-    // output row y: X(y + 1), dZ(y).  An item is published (proxy fence + arrive) once WINFLIGHT - 1
-    // newer ones are in flight, or at the end.
-    const int pt = threadIdx.x;
-    int nx = 0, nd = 0;                           // items issued of each kind
-    int kinds = 0;                                // bit i of the in-flight FIFO: 1 = dZ row
-    int pending = 0;                              // items issued but not yet published
-    int pub_x = 0, pub_d = 0;
-    auto publish_oldest = [&]() {
-      const bool isd = (kinds >> (pending - 1)) & 1;    // oldest at the highest bit
-      fence_proxy_async();
-      if (isd) bar_arrive(&dfull[pub_d++ % wg::DSL]);
-      else bar_arrive(&xfull[pub_x++ % wg::XS]);
-      --pending;
-      kinds &= (1 << pending) - 1;
-    };
-    auto after_issue = [&](bool isd) {
-      cp_async_commit();
-      kinds = (kinds << 1) | (isd ? 1 : 0);
-      ++pending;
-      if (pending >= wg::WINFLIGHT) {
-        cp_async_wait<wg::WINFLIGHT - 1>();       // the oldest pending item has landed
-        publish_oldest();
-      }
-    };
-    auto issue_x = [&](int z, int yw) -> bool {
-      const int slot = nx % wg::XS;
-      if (nx >= wg::XS && !wbar_wait(&xfree[slot], (uint32_t)((nx / wg::XS - 1) & 1), abort, 1, nx, nd)) return false;
-      unsigned char* gb = xring + slot * wg::XGROUP;
+    // Per z-plane segment [yb, ye) of the CTA's rows: X(yb - 1), X(yb), then per output row y: X(y + 1), dZ(y).
+    if (lane == 0) {
+      int nx = 0, nd = 0;                           // items issued of each kind
+      auto issue_x = [&](int z, int yw) -> bool {
+        const int slot = nx % wg::XS;
+        if (nx >= wg::XS && !wbar_wait(&xfree[slot], (uint32_t)((nx / wg::XS - 1) & 1), abort, 1, nx, nd)) return false;
+        bar_expect_tx(&xfull[slot], L::X_TX);
 #pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        const __nv_bfloat16* src = x + (size_t)(((z + d + N - 1) % N) * N + yw) * N * CIN;
-        unsigned char* dst = gb + d * wg::XROW;
-        for (int c = pt; c < KC * N; c += PRODUCERS) {
-          const int kc = c % KC, v = c / KC;
-          cp_async16(dst + kc * wg::CH + v * 16, src + (size_t)v * CIN + kc * 8);
-        }
+        for (int d = 0; d < 3; ++d)
+          tma_load3(xring + slot * L::XGROUP + d * L::XROW, &tm_x, &xfull[slot], 0, 0, ((z + d + N - 1) % N) * N + yw);
+        ++nx;
+        return true;
+      };
+      auto issue_d = [&](int r) -> bool {
+        const int slot = nd % wg::DSL;
+        if (nd >= wg::DSL && !wbar_wait(&dfree[slot], (uint32_t)((nd / wg::DSL - 1) & 1), abort, 2, nd, nx)) return false;
+        bar_expect_tx(&dfull[slot], L::D_TX);
+        unsigned char* dst = dring + slot * L::DROW;
+        tma_load3(dst, &tm_d, &dfull[slot], 0, 0, r);
+        tma_load3(dst - 128, &tm_dend, &dfull[slot], 0, N - L::HALO, r);
+        tma_load3(dst + N * L::DV, &tm_dend, &dfull[slot], 0, 0, r);
+        ++nd;
+        return true;
+      };
+      bool ok = true;
+      for (int r = rg.r0; r < rg.r1 && ok;) {
+        const int z = r / N, yb = r % N;
+        const int ye = (z + 1) * N < rg.r1 ? N : rg.r1 - z * N;
+        ok = issue_x(z, (yb - 1 + N) % N) && issue_x(z, yb);
+        for (int y = yb; y < ye && ok; ++y) ok = issue_x(z, (y + 1) % N) && issue_d(z * N + y);
+        r = z * N + ye;
       }
-      ++nx;
-      after_issue(false);
-      return true;
-    };
-    auto issue_d = [&](int r) -> bool {
-      const int slot = nd % wg::DSL;
-      if (nd >= wg::DSL && !wbar_wait(&dfree[slot], (uint32_t)((nd / wg::DSL - 1) & 1), abort, 2, nd, nx)) return false;
-      const __nv_bfloat16* src = dz + (size_t)r * N * COUT;
-      unsigned char* db = dring + slot * L::DSLOT;
-#pragma unroll
-      for (int sh = 0; sh < 3; ++sh) {               // copy sh holds dZ[(u - dx) mod N] at u, dx = sh - 1
-        unsigned char* dst = db + sh * L::DCOPY;
-        for (int c = pt; c < KCD * N; c += PRODUCERS) {
-          const int kc = c % KCD, u = c / KCD;
-          const int v = (u - (sh - 1) + N) % N;
-          cp_async16(dst + kc * wg::CH + u * 16, src + (size_t)v * COUT + kc * 8);
-        }
+      // after an abort, what is under way lands before the CTA leaves (bounded)
+      if (*abort) {
+        for (int q = nx > wg::XS ? nx - wg::XS : 0; q < nx; ++q)
+          for (long i = 0; i < kWSpin && !bar_try(&xfull[q % wg::XS], (uint32_t)((q / wg::XS) & 1)); ++i) {
+          }
+        for (int q = nd > wg::DSL ? nd - wg::DSL : 0; q < nd; ++q)
+          for (long i = 0; i < kWSpin && !bar_try(&dfull[q % wg::DSL], (uint32_t)((q / wg::DSL) & 1)); ++i) {
+          }
       }
-      ++nd;
-      after_issue(true);
-      return true;
-    };
-    bool ok = true;
-    for (int r = rg.r0; r < rg.r1 && ok && !*abort;) {
-      const int z = r / N, yb = r % N;
-      const int ye = (z + 1) * N < rg.r1 ? N : rg.r1 - z * N;
-      ok = issue_x(z, (yb - 1 + N) % N) && issue_x(z, yb);
-      for (int y = yb; y < ye && ok && !*abort; ++y)
-        ok = issue_x(z, (y + 1) % N) && issue_d(z * N + y);
-      // The segment's last items are published now: the next segment opens with two input groups,
-      // and the second waits for the slot of a group that this segment's last row still reads.
-      cp_async_wait<0>();
-      if (ok && !*abort)
-        while (pending > 0) publish_oldest();
-      r = z * N + ye;
     }
-    cp_async_wait<0>();
-    if (!*abort)
-      while (pending > 0) publish_oldest();
-  } else if (warp == MMA_WARP) {
+  } else if (warp == CONV_MMA_WARP) {
     // ---------------------------------------------------------------- MMA issue
-    const uint64_t a_base = mdesc_mn(saddr(xring), 128, wg::CH);
-    const uint64_t b_base = mdesc_mn(saddr(dring), 128, wg::CH);
+    const uint64_t a_base = mdesc_mn<L::XV>(saddr(xring), L::XROW);
+    const uint64_t b_base = mdesc_mn<L::DV>(saddr(dring) - L::DV, L::DV);   // dx = +1, 0, -1
     constexpr uint32_t idesc = idesc_bf16_mn(128, L::NCOLS);
     int gx = 0, gd = 0;
     bool ok = true;
@@ -665,25 +699,34 @@ __global__ void __launch_bounds__(THREADS, 1) wgrad_tc_kernel(const __nv_bfloat1
       const int z = r / N, yb = r % N;
       const int ye = (z + 1) * N < rg.r1 ? N : rg.r1 - z * N;
       const int nrows = ye - yb;
-      ok = __all_sync(0xFFFFFFFFu, wbar_wait(&xfull[gx % wg::XS], (uint32_t)((gx / wg::XS) & 1), abort, 3, gx, gd)) &&
-           __all_sync(0xFFFFFFFFu, wbar_wait(&xfull[(gx + 1) % wg::XS], (uint32_t)(((gx + 1) / wg::XS) & 1), abort, 3, gx + 1, gd));
+      auto x_here = [&](int g, int tag) {
+        return __all_sync(0xFFFFFFFFu, wbar_wait(&xfull[g % wg::XS], (uint32_t)((g / wg::XS) & 1), abort, tag, g, gd));
+      };
+      auto row_here = [&](int i, int d) {
+        return x_here(gx + i + 2, 4) &&
+               __all_sync(0xFFFFFFFFu, wbar_wait(&dfull[d % wg::DSL], (uint32_t)((d / wg::DSL) & 1), abort, 5, d, gx + i + 2));
+      };
+      ok = x_here(gx, 3) && x_here(gx + 1, 3) && row_here(0, gd);
       for (int i = 0; i < nrows && ok; ++i) {
-        const int gn = gx + i + 2;
-        ok = __all_sync(0xFFFFFFFFu, wbar_wait(&xfull[gn % wg::XS], (uint32_t)((gn / wg::XS) & 1), abort, 4, gn, gd)) &&
-             __all_sync(0xFFFFFFFFu, wbar_wait(&dfull[gd % wg::DSL], (uint32_t)((gd / wg::DSL) & 1), abort, 5, gd, gn));
-        if (!ok) break;
         tc_after();
-        const uint64_t bd = b_base + (uint64_t)((gd % wg::DSL) * (L::DSLOT / 16));
+        const uint64_t bd = b_base + (uint64_t)((gd % wg::DSL) * (L::DROW / 16));
+        bool next_ok = true;
 #pragma unroll
         for (int dyi = 0; dyi < 3; ++dyi) {
-          const uint64_t ad = a_base + (uint64_t)(((gx + i + dyi) % wg::XS) * (wg::XGROUP / 16));
+          // the waits for the next row's items stand before the last dy, beside the MMAs in the queue
+          if (dyi == 2 && i + 1 < nrows) {
+            next_ok = row_here(i + 1, gd + 1);
+            tc_after();
+          }
+          const uint64_t ad = a_base + (uint64_t)(((gx + i + dyi) % wg::XS) * (L::XGROUP / 16));
           const uint32_t dcol = tmem + (uint32_t)(dyi * L::NCOLS);
 #pragma unroll
-          for (int ks = 0; ks < N / 16; ++ks) mma_acc(dcol, ad + (uint64_t)(ks * 16), bd + (uint64_t)(ks * 16), idesc);
+          for (int ks = 0; ks < N / 16; ++ks) mma_acc(dcol, ad + (uint64_t)(ks * L::XV), bd + (uint64_t)(ks * L::DV), idesc);
         }
         mma_commit(&dfree[gd % wg::DSL]);           // this dZ row is not read again
         mma_commit(&xfree[(gx + i) % wg::XS]);      // nor is input group y - 1
         ++gd;
+        ok = next_ok;
       }
       if (!ok) break;
       mma_commit(&xfree[(gx + nrows) % wg::XS]);    // groups ye - 1 and ye end with the segment
@@ -712,9 +755,11 @@ __global__ void __launch_bounds__(THREADS, 1) wgrad_tc_kernel(const __nv_bfloat1
           float v[COUT];
           const uint32_t ta = tmem + lanes + (uint32_t)(dyi * L::NCOLS + c0);
           if (COUT == 32) tmem_ld32(ta, v); else tmem_ld16(ta, v);
-          float* row = dst + ((size_t)dyi * 128 + m) * L::NCOLS + c0;
+          if (m <= L::ONES) {                       // rows past the ones row's first are not read
+            float* row = dst + ((size_t)dyi * 128 + m) * L::NCOLS + c0;
 #pragma unroll
-          for (int c = 0; c < COUT; c += 4) *reinterpret_cast<float4*>(row + c) = make_float4(v[c], v[c + 1], v[c + 2], v[c + 3]);
+            for (int c = 0; c < COUT; c += 4) *reinterpret_cast<float4*>(row + c) = make_float4(v[c], v[c + 1], v[c + 2], v[c + 3]);
+          }
         }
       }
     }
@@ -729,28 +774,58 @@ __global__ void __launch_bounds__(THREADS, 1) wgrad_tc_kernel(const __nv_bfloat1
   }
 }
 
-// dW[27][COUT][CIN] and db[COUT] from the per-CTA partials [cta][dy][(dz, ci) | ones][(dx, co)],
-// summed over CTAs in a fixed order.
+// dW[27][COUT][CIN] and db[COUT] from the per-CTA partials [cta][dy][(dz, ci) | ones][(dx, co)], summed
+// over CTAs in a fixed order.  A block takes 32 neighbouring columns of one accumulator row, eight groups
+// of CTAs beside each other: contiguous reads, ~20 in flight per thread.  A thread per element of dW, each
+// reading its 152 partials one line apart, took 42 us; this 8 us (14.5 MB).
 template <int CIN, int COUT>
-__global__ void wgrad_tc_reduce(const float* __restrict__ partials, int ctas, float* __restrict__ dw,
-                                float* __restrict__ db) {
-  constexpr int NCOLS = 3 * COUT, PER = 3 * 128 * NCOLS, NW = 27 * COUT * CIN;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < NW + COUT; i += gridDim.x * blockDim.x) {
-    int dyi, m, n;
-    if (i < NW) {
-      const int t = i / (COUT * CIN), co = (i / CIN) % COUT, ci = i % CIN;
-      dyi = (t / 3) % 3;
-      m = (t / 9) * 32 + ci;
-      n = (t % 3) * COUT + co;
-    } else {
-      dyi = 1;
-      m = 96;                                      // the ones row
-      n = COUT + (i - NW);                         // the unshifted dZ copy
-    }
-    float s = 0.f;
-    for (int c = 0; c < ctas; ++c) s += partials[(size_t)c * PER + ((size_t)dyi * 128 + m) * NCOLS + n];
-    if (i < NW) dw[i] = s; else db[i - NW] = s;
+__global__ void __launch_bounds__(256) wgrad_tc_reduce(const float* __restrict__ partials, int ctas, float* __restrict__ dw,
+                                                       float* __restrict__ db) {
+  using L = WLayout<CIN, COUT>;
+  constexpr int NCOLS = L::NCOLS, PER = 3 * 128 * NCOLS, ROWS = L::ONES + 1;
+  __shared__ float part[8][32];
+  const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
+  const int e = blockIdx.x * 32 + lane;               // element of [3][ROWS][NCOLS]
+  const bool here = e < 3 * ROWS * NCOLS;
+  const int n = e % NCOLS, m = (e / NCOLS) % ROWS, dyi = e / (NCOLS * ROWS);
+  const float* src = partials + ((size_t)dyi * 128 + m) * NCOLS + n;
+  const int per = (ctas + 7) / 8, c1 = min(ctas, (g + 1) * per);
+  float s = 0.f;
+  if (here) {
+#pragma unroll 20
+    for (int c = g * per; c < c1; ++c) s += __ldcg(src + (size_t)c * PER);
   }
+  part[g][lane] = s;
+  __syncthreads();
+  if (g || !here) return;
+  s = 0.f;
+#pragma unroll
+  for (int q = 0; q < 8; ++q) s += part[q][lane];
+  const int dx = 2 - n / COUT, co = n % COUT;         // column blocks: dx = +1, 0, -1
+  if (m < L::ONES) dw[((size_t)((m / CIN) * 9 + dyi * 3 + dx) * COUT + co) * CIN + m % CIN] = s;
+  else if (dyi == 1 && dx == 1) db[co] = s;           // the ones row, the unshifted dZ
+}
+
+// TMA descriptor of a channels-last box [row = z N + y][x][cin]: boxes of `voxels` voxels of one row, swizzled
+// over a voxel's bytes
+bool row_map(CUtensorMap* m, const void* base, int cin, int voxels) {
+  static PFN_cuTensorMapEncodeTiled_v12000 enc = nullptr;
+  static std::once_flag once;
+  std::call_once(once, [] {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &f, 12000, cudaEnableDefault, &q) == cudaSuccess &&
+        q == cudaDriverEntryPointSuccess)
+      enc = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(f);
+  });
+  if (!enc) return false;
+  cuuint64_t dims[3] = {(cuuint64_t)cin, (cuuint64_t)N, (cuuint64_t)N * N};
+  cuuint64_t strides[2] = {(cuuint64_t)cin * 2, (cuuint64_t)N * cin * 2};
+  cuuint32_t box[3] = {(cuuint32_t)cin, (cuuint32_t)voxels, 1u};
+  cuuint32_t estr[3] = {1, 1, 1};
+  return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
+             CU_TENSOR_MAP_INTERLEAVE_NONE, cin == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B,
+             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 template <int CIN, int COUT>
@@ -774,10 +849,16 @@ int launch_wgrad(const void* x, const void* dz, float* dw, float* db, float* ws,
     *err = "tcgen05 wgrad: workspace needs " + std::to_string(need) + " bytes";
     return ES_E_ARG;
   }
-  kern<<<sms, THREADS, L::BYTES, s>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)dz, ws);
+  CUtensorMap mx, md, me;
+  if (!row_map(&mx, x, CIN, N) || !row_map(&md, dz, COUT, N) || !row_map(&me, dz, COUT, L::HALO)) {
+    *err = "tcgen05 wgrad: cuTensorMapEncodeTiled failed";
+    return ES_E_CUDA;
+  }
+  kern<<<sms, wg::WG_THREADS, L::BYTES, s>>>(mx, md, me, ws);
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess) {
-    wgrad_tc_reduce<CIN, COUT><<<64, 256, 0, s>>>(ws, sms, dw, db);
+    constexpr int ELEMS = 3 * (L::ONES + 1) * L::NCOLS;
+    wgrad_tc_reduce<CIN, COUT><<<(ELEMS + 31) / 32, 256, 0, s>>>(ws, sms, dw, db);
     e = cudaGetLastError();
   }
   if (e != cudaSuccess) {
@@ -804,8 +885,12 @@ int launch(const void* in, const void* w, const float* bias, void* out, const vo
     configured |= 1u << (dev & 31);
   }
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  kern<<<sms, THREADS, L::BYTES, s>>>((const __nv_bfloat16*)in, (const __nv_bfloat16*)w, bias, out,
-                                      (const __nv_bfloat16*)mask);
+  CUtensorMap row, end;
+  if (!row_map(&row, in, CIN, N) || !row_map(&end, in, CIN, L::HALO)) {
+    *err = "tcgen05 conv: cuTensorMapEncodeTiled failed";
+    return ES_E_CUDA;
+  }
+  kern<<<sms, CONV_THREADS, L::BYTES, s>>>(row, end, (const __nv_bfloat16*)w, bias, out, (const __nv_bfloat16*)mask);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
     *err = std::string("tcgen05 conv launch: ") + cudaGetErrorString(e);
