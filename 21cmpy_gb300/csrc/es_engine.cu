@@ -96,10 +96,8 @@ struct es_plan {
   unsigned* counters = nullptr;     // [0] reductions, [2] error word, [16..63] P(k) groups
   float* stats = nullptr;           // [max_radii + 2][4]: sum, mean, norm, centres found (unsigned)
   RadDev* rad = nullptr;
-  int* thr = nullptr;
   // pinned host staging for per-call parameter uploads
   RadDev* h_rad = nullptr;
-  int* h_thr = nullptr;
   std::vector<RadDev> hr;           // this call's per-radius parameters (kernel arguments by value)
   cudaEvent_t staged = nullptr;     // last upload from the staging buffers
   size_t partial_floats = 0;
@@ -139,7 +137,7 @@ constexpr int kStatsStride = 4;
 size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
 struct Layout {
-  size_t X, Xnyq, T, Tnyq, T2, Tnyq2, tw, dR0, dR1, flags, centres, wtab, partials, counters, stats, rad, thr, total;
+  size_t X, Xnyq, T, Tnyq, T2, Tnyq2, tw, dR0, dR1, flags, centres, wtab, partials, counters, stats, rad, total;
 };
 
 Layout layout(int n, int max_radii, size_t partial_floats) {
@@ -164,7 +162,6 @@ Layout layout(int n, int max_radii, size_t partial_floats) {
   L.counters = take(256);
   L.stats = take((size_t)(max_radii + 2) * kStatsStride * 4);
   L.rad = take((size_t)max_radii * sizeof(RadDev));
-  L.thr = take(es::PK_MAX_BINS * 4);
   L.total = off;
   return L;
 }
@@ -585,7 +582,7 @@ void prof_end(es_plan* p, int slot, cudaStream_t s) {
   if (slot >= 0) cudaEventRecord(p->prof_events[2 * slot + 1], s);
 }
 
-int run_op(es_plan* p, int op, es::OpArgs a, int grid, cudaStream_t s) {
+int run_op(es_plan* p, int op, es::OpArgs& a, int grid, cudaStream_t s) {   // OP_COL_Z_FWD_PK: an es::PkArgs
   a.grid = grid;
   a.pdl = uses_pdl(p);
   a.stall = (p->stall == ES_STALL_COL_Z_INV && op == es::OP_COL_Z_INV_FILTER) ||
@@ -770,12 +767,10 @@ int es_plan_create(int n, double box_len, int max_radii, es_plan** out) {
   p->counters = (unsigned*)(b + L.counters);
   p->stats = (float*)(b + L.stats);
   p->rad = (RadDev*)(b + L.rad);
-  p->thr = (int*)(b + L.thr);
   p->err = p->counters + 2;
   if (int rc = encode_maps(p)) return cleanup(rc);
   if (int rc = encode_warp_maps(p)) return cleanup(rc);
-  if (cudaMallocHost(&p->h_rad, sizeof(RadDev) * max_radii) != cudaSuccess ||
-      cudaMallocHost(&p->h_thr, sizeof(int) * es::PK_MAX_BINS) != cudaSuccess)
+  if (cudaMallocHost(&p->h_rad, sizeof(RadDev) * max_radii) != cudaSuccess)
     return cleanup(fail(ES_E_NOMEM, "es_plan_create: pinned staging allocation failed"));
   if (cudaEventCreateWithFlags(&p->staged, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&p->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
@@ -808,7 +803,6 @@ int es_plan_destroy(es_plan* p) {
   if (p->aux) cudaStreamSynchronize(p->aux);
   if (p->base) cudaFree(p->base);
   if (p->h_rad) cudaFreeHost(p->h_rad);
-  if (p->h_thr) cudaFreeHost(p->h_thr);
   if (p->staged) cudaEventDestroy(p->staged);
   for (cudaEvent_t e : {p->ev_fork, p->ev_col[0], p->ev_col[1], p->ev_row[0], p->ev_row[1]})
     if (e) cudaEventDestroy(e);
@@ -1036,11 +1030,7 @@ int es_power_spectrum(es_plan* p, const float* dT, const float* ave, const int* 
     if (thr[b] < thr[b - 1]) return fail(ES_E_ARG, "es_power_spectrum: k^2 thresholds must be non-decreasing");
   DeviceGuard g(p->device);
   cudaStream_t s = (cudaStream_t)stream;
-  int rc = reuse_staging(p);
-  if (rc) return rc;
-  std::memcpy(p->h_thr, thr, sizeof(int) * nbins);
-  ES_CUDA(cudaMemcpyAsync(p->thr, p->h_thr, sizeof(int) * nbins, cudaMemcpyHostToDevice, s));
-  ES_CUDA(cudaEventRecord(p->staged, s));
+  int rc = 0;
   const double L = (double)(float)p->box_len;
   es::OpArgs a = base_args(p);
   a.rin = reinterpret_cast<const float2*>(dT);
@@ -1053,12 +1043,14 @@ int es_power_spectrum(es_plan* p, const float* dT, const float* ave, const int* 
   a.cin = p->T; a.cout = p->T; a.cout_nyq = p->Tnyq;
   set_maps(a, p, SPEC_T, SPEC_T, false, uses_col_warp(p, false));
   if ((rc = run_op(p, es::OP_COL_Y_FWD, a, grid_col_y(p), s))) return rc;
-  a = base_args(p);
-  a.cin = p->T; a.cin_nyq = p->Tnyq;
-  set_maps(a, p, SPEC_T, SPEC_T, true, false);
-  a.thr = p->thr; a.nbins = nbins; a.dk = p->dk; a.volume = (float)(L * L * L);
-  a.pk_out = out;
-  return run_op(p, es::OP_COL_Z_FWD_PK, a, grid_col_z(p, true), s);
+  es::PkArgs b;
+  static_cast<es::OpArgs&>(b) = base_args(p);
+  b.cin = p->T; b.cin_nyq = p->Tnyq;
+  set_maps(b, p, SPEC_T, SPEC_T, true, false);
+  std::memcpy(b.thr, thr, sizeof(int) * nbins);
+  b.nbins = nbins; b.dk = p->dk; b.volume = (float)(L * L * L);
+  b.pk_out = out;
+  return run_op(p, es::OP_COL_Z_FWD_PK, b, grid_col_z(p, true), s);
 }
 
 int es_fft_r2c(es_plan* p, const float* in, void* out, void* stream) {

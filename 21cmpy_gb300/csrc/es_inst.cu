@@ -16,8 +16,8 @@ namespace es {
 // One static record per kernel (the template argument is the kernel itself) and device: opt in to
 // more than 48 KB of dynamic shared memory once, and remember how many CTAs of it fit on the
 // device at once (registers included), so a persistent grid never exceeds one resident wave.
-template <auto Kernel>
-static cudaError_t launch(int smem, const OpArgs& a, int threads, cudaStream_t s) {
+template <auto Kernel, class Args>
+static cudaError_t launch(int smem, const Args& a, int threads, cudaStream_t s) {
   static unsigned configured = 0u;
   static int resident[32];
   int dev = 0;
@@ -50,7 +50,8 @@ static cudaError_t launch(int smem, const OpArgs& a, int threads, cudaStream_t s
 }
 
 template <int N, int MODE, int RS>
-static cudaError_t launch_col_tma(const OpArgs& a, cudaStream_t s) {
+static cudaError_t launch_col_tma(const OpArgs& base, cudaStream_t s) {
+  const auto& a = static_cast<const typename ColArgs<MODE>::type&>(base);
   if (a.col_tile == 1) return launch<col_tma<N, MODE, 1, RS>>(TmaSmem<N, MODE, 1>::bytes, a, ColTile<N, 1>::T, s);
   if (a.col_tile == 2) return launch<col_tma<N, MODE, 2, RS>>(TmaSmem<N, MODE, 2>::bytes, a, ColTile<N, 2>::T, s);
   // tile shape 0 with the large radices is the warp-per-columns form at the sizes that have it
@@ -61,7 +62,9 @@ static cudaError_t launch_col_tma(const OpArgs& a, cudaStream_t s) {
 // The per-radius column passes also come with the small-radix schedule (ES_OPT_COL_RADIX).
 template <int N, int MODE>
 static cudaError_t launch_col(const OpArgs& a, cudaStream_t s) {
-  if (a.variant == 0) return launch<col_pass<N, MODE>>(ColSmem<N, MODE>::bytes, a, ColCfg<N>::T, s);
+  if (a.variant == 0)
+    return launch<col_pass<N, MODE>>(ColSmem<N, MODE>::bytes, static_cast<const typename ColArgs<MODE>::type&>(a),
+                                     ColCfg<N>::T, s);
   if constexpr (ColW<N>::TI > 0 && MODE != COL_Z_FWD_PK) {
     if (a.col_warp) return launch<col_warp<N, MODE>>(ColWSmem<N, MODE>::bytes, a, ColWSmem<N, MODE>::T, s);
   }

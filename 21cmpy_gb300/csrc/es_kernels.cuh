@@ -85,7 +85,6 @@ struct OpArgs {
   float fc_mean;                  // mean collapse fraction (normalisation target)
   int normalize;                  // rescale fcoll by fc_mean / <fcoll>
   // P(k)
-  const int* thr;                 // integer k^2 thresholds per bin
   int nbins;
   float dk;
   float volume;
@@ -101,6 +100,12 @@ struct OpArgs {
 // filter tables behind the tail of the kernel before: a 64^3 box (~95 short launches) 603 -> 371 us.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// Arguments of the P(k) binning pass: the bins' integer k^2 thresholds come by value, so a call needs no
+// staging buffer, copy or wait for the last call's copy.
+struct PkArgs : OpArgs { int thr[PK_MAX_BINS]; };
+template <int MODE> struct ColArgs { typedef OpArgs type; };
+template <> struct ColArgs<COL_Z_FWD_PK> { typedef PkArgs type; };
 
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
@@ -551,7 +556,7 @@ template <int N, int MODE> struct ColSmem {
 };
 
 template <int N, int MODE>
-__global__ void __launch_bounds__(ColCfg<N>::T) col_pass(OpArgs a) {
+__global__ void __launch_bounds__(ColCfg<N>::T) col_pass(const __grid_constant__ typename ColArgs<MODE>::type a) {
   constexpr int M = N / 2;
   constexpr int TI = ColCfg<N>::TI, T = ColCfg<N>::T;
   constexpr bool INV = (MODE == COL_Z_INV_FILTER || MODE == COL_Y_INV || MODE == COL_Z_INV);
@@ -571,7 +576,7 @@ __global__ void __launch_bounds__(ColCfg<N>::T) col_pass(OpArgs a) {
   __shared__ float sred[T / 32];
 
   for (int i = threadIdx.x; i < N; i += T) tw[i] = a.tw[i];
-  if (MODE == COL_Z_FWD_PK) {
+  if constexpr (MODE == COL_Z_FWD_PK) {
     for (int i = threadIdx.x; i < (T / 32) * PK_MAX_BINS * 3; i += T) bins[i] = 0.f;
     for (int i = threadIdx.x; i < a.nbins; i += T) sthr[i] = a.thr[i];
   }

@@ -233,7 +233,7 @@ template <int N, int MODE, int V> struct TmaSmem {
 };
 
 template <int N, int MODE, int V, int RS = 0>
-__global__ void __launch_bounds__(ColTile<N, V>::T, ColTile<N, V>::MINB) col_tma(const __grid_constant__ OpArgs a) {
+__global__ void __launch_bounds__(ColTile<N, V>::T, ColTile<N, V>::MINB) col_tma(const __grid_constant__ typename ColArgs<MODE>::type a) {
   constexpr int M = N / 2;
   constexpr int TI = ColTile<N, V>::TI, T = ColTile<N, V>::T;
   constexpr bool INV = (MODE == COL_Z_INV_FILTER || MODE == COL_Y_INV || MODE == COL_Z_INV);
@@ -272,7 +272,7 @@ __global__ void __launch_bounds__(ColTile<N, V>::T, ColTile<N, V>::MINB) col_tma
       issue_tile_load<N, MODE, V>(a, seq.at(s, &reuse_w), s ? S1 : S0, &bars[s], stall_bytes(a.stall, s));
     if (!a.early) pdl_trigger();
   }
-  if (MODE == COL_Z_FWD_PK) {
+  if constexpr (MODE == COL_Z_FWD_PK) {
     for (int i = threadIdx.x; i < (T / 32) * PK_MAX_BINS * 3; i += T) bins[i] = 0.f;
     for (int i = threadIdx.x; i < a.nbins; i += T) sthr[i] = a.thr[i];
   }

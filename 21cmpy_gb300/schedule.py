@@ -158,10 +158,14 @@ def pk_k2_thresholds(n: int, box_len: float, edges: np.ndarray) -> np.ndarray:
     """
     dk = float(delta_k(box_len))
     kmax2 = 3 * (n // 2) ** 2
-    out = np.empty(len(edges), dtype=np.int64)
-    for b, e in enumerate(np.asarray(edges, dtype=np.float64)):
-        m = int(math.floor((e / dk) ** 2)) + 2
-        while m >= 0 and dk * math.sqrt(m) > e:
-            m -= 1
-        out[b] = min(m, kmax2)
-    return out.astype(np.int32)
+    e = np.asarray(edges, dtype=np.float64)
+    if not np.isfinite(e).all():
+        raise ValueError("bin edges must be finite")
+    m = np.minimum(np.floor((e / dk) ** 2), kmax2 + 8.0).astype(np.int64) + 2
+    m[e < 0] = -1
+    while True:                                     # at most a few steps: down to the last m with dk sqrt(m) <= edge
+        over = (m >= 0) & (dk * np.sqrt(np.maximum(m, 0)) > e)
+        if not over.any():
+            break
+        m[over] -= 1
+    return np.minimum(m, kmax2).astype(np.int32)
