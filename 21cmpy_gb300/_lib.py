@@ -82,6 +82,7 @@ _PROTOS = {
     "es_delta_T_noalloc": (C.c_int, [C.c_int, C.c_void_p, C.c_void_p, C.c_float, C.c_void_p, C.c_void_p, C.c_void_p]),
     "es_power_spectrum": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.POINTER(C.c_int), C.c_int, C.c_int,
                                     C.c_void_p, C.c_void_p]),
+    "es_smooth": (C.c_int, [C.c_void_p, C.POINTER(C.c_float), C.c_int, C.c_void_p, C.c_void_p]),
     "es_fft_r2c": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]),
     "es_fft_c2r": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]),
     "es_fft_c2r_scaled": (C.c_int, [C.c_void_p, C.c_void_p, C.c_float, C.c_void_p, C.c_void_p]),

@@ -430,6 +430,25 @@ __global__ void erfc_selftest_kernel(const float* x, float* fast, float* lib, in
   }
 }
 
+// The real-space top hat times a spectrum, in the plan's layout.  A pass of its own and not the radius
+// loop's filtered z inverse: there the product is contracted into the first butterfly, and the smoothed
+// fields, which the surrogate rounds to BF16, would not keep their bits.  Bound by L2 at 128^3 (9 us; the
+// layout conversions, copy and scaling it replaces took 25 us a radius).
+__global__ void window_kernel(const float2* in, const float2* in_nyq, float2* out, float2* out_nyq, int n, float dk, float R) {
+  es::pdl_wait();
+  es::pdl_trigger();
+  const int m = n / 2, lane = threadIdx.x & 31, step = gridDim.x * (blockDim.x / 32);
+  for (int row = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5); row < n * n; row += step) {
+    const int k0 = row / n, k1 = row - k0 * n, w0 = k0 > m ? k0 - n : k0, w1 = k1 > m ? k1 - n : k1;
+    const int ck2 = w0 * w0 + w1 * w1;
+    for (int x = lane; x <= m; x += 32) {
+      const float W = es::filter_weight(ck2 + x * x, dk, R, 0x7fffffff, 0, 0);
+      const float2 v = x < m ? in[(size_t)row * m + x] : in_nyq[row];
+      (x < m ? out[(size_t)row * m + x] : out_nyq[row]) = make_float2(v.x * W, v.y * W);
+    }
+  }
+}
+
 // numpy rfftn layout (n, n, n/2+1)  <->  main (n, n, n/2) + nyq (n, n)
 __global__ void to_std_kernel(const float2* mainp, const float2* nyq, float2* out, int n) {
   const int m = n / 2;
@@ -1003,6 +1022,21 @@ int es_ionize(es_plan* p, const es_ionize_params* prm, float* out, float* nf, vo
       inv_zeta, prm->output, reinterpret_cast<float2*>(out), p->partials, p->counters, nf, inv_n3);
   prof_end(p, slot, s);
   ES_CUDA(le);
+  return ES_OK;
+}
+
+int es_smooth(es_plan* p, const float* R, int count, float* out, void* stream) {
+  if (!p || count < 0 || (count > 0 && (!R || !out))) return fail(ES_E_ARG, "es_smooth: bad arguments");
+  if (p->fft_only) return fail(ES_E_UNSUPPORTED, "es_smooth: the plan is for transforms alone");
+  DeviceGuard g(p->device);
+  cudaStream_t s = (cudaStream_t)stream;
+  const size_t N3 = (size_t)p->n * p->n * p->n;
+  for (int j = 0; j < count; ++j) {
+    const cudaError_t e = launch_pdl(uses_pdl(p), window_kernel, p->sms * 8, 256, s, (const float2*)p->X, (const float2*)p->Xnyq,
+                                     p->T, p->Tnyq, p->n, p->dk, R[j]);
+    if (e != cudaSuccess) return fail(ES_E_CUDA, "es_smooth: launch failed: %s", cudaGetErrorString(e));
+    if (int rc = inverse_from(p, SPEC_T, (float)(1.0 / (double)N3), out + j * N3, s)) return rc;
+  }
   return ES_OK;
 }
 

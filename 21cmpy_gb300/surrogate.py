@@ -154,24 +154,19 @@ _smooth_plans = {}
 
 def smoothed_fields(delta: torch.Tensor, radii_cells) -> torch.Tensor:
     """The density smoothed with the real-space top hat W(kR) at each radius (in cells): one forward
-    transform, then per radius the window (``ic_shape``, the excursion set's filter) and an inverse
-    transform, all on the engine's kernels.  Returns float32 [len(radii), n, n, n]."""
+    transform, then per radius the window and an inverse transform (``es_smooth``).
+    Returns float32 [len(radii), n, n, n]."""
     from .engine import ExcursionSetPlan
     n = delta.shape[0]
     key = (n, str(delta.device))
     if key not in _smooth_plans:
         _smooth_plans[key] = ExcursionSetPlan(n, float(n), max_radii=1, device=delta.device)   # lengths in cells
     plan = _smooth_plans[key]
-    lib = _lib.load()
     out = torch.empty((len(radii_cells), n, n, n), dtype=torch.float32, device=delta.device)
+    radii = (C.c_float * len(radii_cells))(*[float(R) for R in radii_cells])
     with torch.cuda.device(delta.device):
-        X = plan.fft_r2c(delta)
-        Y = torch.empty_like(X)
-        for j, R in enumerate(radii_cells):
-            rc = lib.ic_shape(n, C.c_float(float(n)), _p(X), -1, 0, C.c_float(float(R)), 0, _p(Y), _stream())
-            _lib.check("ic_shape", rc, lib)
-            out[j] = plan.fft_c2r(Y)
-        out *= 1.0 / float(n) ** 3
+        plan.forward(delta)
+        _lib.check("es_smooth", plan.lib.es_smooth(plan.handle, radii, len(radii_cells), _p(out), _stream()), plan.lib)
     return out
 
 

@@ -148,6 +148,11 @@ int es_delta_T_noalloc(int n, const float* xH, const float* delta, float const_f
 int es_power_spectrum(es_plan* plan, const float* dT, const float* ave, const int* k2_thresholds,
                       int nbins, int dimensional, float* out, void* stream);
 
+/* Copies of the last es_forward's box smoothed with the real-space top hat at radii R[0..count)
+ * (lengths in units of the plan's BOX_LEN's), normalised: out[j], device float n^3 each, one after
+ * another. */
+int es_smooth(es_plan* plan, const float* R, int count, float* out, void* stream);
+
 /* Plain 3-D transforms in numpy's rfftn layout (n, n, n/2 + 1), for testing the FFT passes:
  * forward unnormalised; inverse unnormalised (numpy irfftn times n^3).  Use the plan's
  * scratch spectrum, so they invalidate the last es_forward. */
