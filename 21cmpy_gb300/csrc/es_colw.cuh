@@ -27,11 +27,16 @@ template <> struct ColW<512> { static constexpr int TI = 8,  CPW = 2, NG = 3, NB
 
 template <int N, int MODE> struct ColWSmem {
   static constexpr int TI = ColW<N>::TI, CPW = ColW<N>::CPW;
-  static constexpr int NBUF = ColW<N>::NBUF;
+  // z forward + binning: the warps' bins take the place of a tile (nothing is stored, so that a buffer is
+  // refilled as soon as its tile is binned).  512^3: 420 us in the CTA-wide form, 282 us here (the plain
+  // pass takes 190 us); delta_T and P(k) of a 256^3 box with 100 bins: 155 -> 150 us
+  static constexpr int NBUF = ColW<N>::NBUF - (MODE == COL_Z_FWD_PK ? 1 : 0);
   static constexpr int WPT = TI ? TI / CPW : 1, NW = ColW<N>::NG * WPT, T = 32 * (NW + 1);
   static constexpr int tile = N * TI * 8;
-  static constexpr int wts = MODE == COL_Z_INV_FILTER ? NW * CPW * (N / 2 + 1) * 4 : 0;   // per-warp filter weights
-  // [NBUF tiles | 2 NBUF mbarriers | twiddles by stage | filter weights] after aligning the base to 1024
+  // per-warp filter weights, or per-warp bins and the thresholds
+  static constexpr int wts = MODE == COL_Z_INV_FILTER ? NW * CPW * (N / 2 + 1) * 4
+                             : MODE == COL_Z_FWD_PK   ? (NW * 3 + 1) * PK_MAX_BINS * 4 : 0;
+  // [NBUF tiles | 2 NBUF mbarriers | twiddles by stage | filter weights or bins] after aligning the base to 1024
   static constexpr int bytes = NBUF * tile + 2 * NBUF * 8 + N * 8 + wts + 1024;
 };
 
@@ -44,7 +49,7 @@ template <int N, int MODE> struct ColWSmem {
 struct ColWTile { int plane, c; bool nyq; };
 template <int N, int MODE> struct ColWSeq {
   static constexpr int TI = ColW<N>::TI, CPR = (N / 2) / TI, NG = ColW<N>::NG;
-  static constexpr bool ZPASS = MODE == COL_Z_FWD || MODE == COL_Z_INV_FILTER || MODE == COL_Z_INV;
+  static constexpr bool ZPASS = MODE == COL_Z_FWD || MODE == COL_Z_INV_FILTER || MODE == COL_Z_INV || MODE == COL_Z_FWD_PK;
   static constexpr bool PAIRS = MODE == COL_Z_INV_FILTER;
   static constexpr int NPAIR = (N / 2 - 1) * CPR, NREST = 2 * CPR + N / TI;
   static constexpr int NTILES = N * CPR + (ZPASS ? N / TI : 0);
@@ -186,12 +191,13 @@ template <int N> struct WarpFft {
 };
 
 template <int N, int MODE>
-__global__ void __launch_bounds__(ColWSmem<N, MODE>::T, 1) col_warp(const __grid_constant__ OpArgs a) {
+__global__ void __launch_bounds__(ColWSmem<N, MODE>::T, 1) col_warp(const __grid_constant__ typename ColArgs<MODE>::type a) {
   using SM = ColWSmem<N, MODE>;
   using F = WarpFft<N>;
   constexpr int M = N / 2, TI = SM::TI, CPW = SM::CPW, WPT = SM::WPT, NBUF = SM::NBUF, ROWB = TI * 8;
   constexpr int BOX = N < 256 ? N : 256;
   static_assert(NBUF >= 2, "a buffer is refilled only after the next tile's store is on its way");
+  constexpr bool PK = MODE == COL_Z_FWD_PK;
   constexpr bool INV = MODE == COL_Z_INV_FILTER || MODE == COL_Y_INV || MODE == COL_Z_INV;
   constexpr bool ZPASS = ColWSeq<N, MODE>::ZPASS;
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -229,6 +235,11 @@ __global__ void __launch_bounds__(ColWSmem<N, MODE>::T, 1) col_warp(const __grid
     fence_async_smem();
   }
   F::load_twiddles(tws, a.tw, threadIdx.x, SM::T);
+  int* sthr = reinterpret_cast<int*>(wts + SM::NW * 3 * PK_MAX_BINS);
+  if constexpr (PK) {
+    for (int i = threadIdx.x; i < SM::NW * 3 * PK_MAX_BINS; i += SM::T) wts[i] = 0.f;
+    for (int i = threadIdx.x; i < a.nbins; i += SM::T) sthr[i] = a.thr[i];
+  }
   if (!a.early) pdl_wait();
   if (threadIdx.x == 32 * SM::NW) {
     for (int it = 0; it < NBUF && it < seq.count; ++it) load(it);
@@ -242,6 +253,10 @@ __global__ void __launch_bounds__(ColWSmem<N, MODE>::T, 1) col_warp(const __grid
       int loaded = seq.count < NBUF ? seq.count : NBUF;
       for (int it = 0; it < seq.count; ++it) {
         if (!colw_wait(&done[it % NBUF], (uint32_t)((it / NBUF) & 1), a, abort)) break;
+        if (PK) {
+          if (loaded < seq.count) load(loaded++);
+          continue;
+        }
         if (a.early && it == 0) {
           pdl_wait();
           pdl_trigger();
@@ -270,6 +285,10 @@ __global__ void __launch_bounds__(ColWSmem<N, MODE>::T, 1) col_warp(const __grid
       if (a.early) pdl_wait();                           // also where this CTA has stored nothing
       bulk_wait0();
     }
+    if constexpr (PK) {
+      __syncwarp();
+      pk_finish<SM::T, SM::NW>(wts, a);
+    }
     return;
   }
 
@@ -291,11 +310,20 @@ __global__ void __launch_bounds__(ColWSmem<N, MODE>::T, 1) col_warp(const __grid
     if (lane < CPW) put(lane, M);
     __syncwarp();
   };
+  // meets the group's warps; true if all of them say so (they leave an aborted pass together)
+  auto group_agrees = [&](int g, bool mine) {
+    int r;
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.s32 p, %1, 0;\n\tbar.red.and.pred q, %2, %3, p;\n\tselp.s32 %0, 1, 0, q;\n\t}"
+                 : "=r"(r) : "r"((int)mine), "r"(g + 1), "n"(32 * WPT) : "memory");
+    return r != 0;
+  };
   // transforms the CTA's it-th tile; false: aborted
   auto transform = [&](int it, const ColWTile& t) {
     unsigned char* buf = base + (it % NBUF) * SM::tile;
     const bool ok = colw_wait(&full[it % NBUF], (uint32_t)((it / NBUF) & 1), a, abort);
-    if (!__all_sync(0xffffffffu, ok)) return false;
+    const bool all_ok = __all_sync(0xffffffffu, ok);
+    if (PK && !all_ok) return group_agrees(group, false);
+    if (!all_ok) return false;
     if (MODE == COL_Z_INV_FILTER) {
       F::template stage<0, INV>(buf, piece0, tws, [&](int col, int k, bool upper, float2 v) {
         return cscale(v, w[col * (M + 1) + (upper ? N - k : k)]);
@@ -332,6 +360,18 @@ __global__ void __launch_bounds__(ColWSmem<N, MODE>::T, 1) col_warp(const __grid
         a.cout_nyq[(size_t)t.plane * N + j] = bv[q];
       }
     }
+    if constexpr (PK) {
+      // all of the group's columns, TI neighbouring threads on a row: a warp sees few values of |kz| and so
+      // few bins (its own columns from end to end would be all bins: 131 us at 256^3 with 100 bins)
+      if (!group_agrees(group, true)) return false;
+      constexpr int GT = 32 * WPT;
+      const int tid = wt * 32 + lane, col = tid % TI, kx = t.c * TI + col;
+      const int ck2 = t.nyq ? wrap2<N>(kx) + M * M : wrap2<N>(t.plane) + kx * kx;
+      float* wb = wts + warp * 3 * PK_MAX_BINS;
+      pk_bin_segment<N, (M * TI + GT - 1) / GT>(
+          [&](int k) { return *reinterpret_cast<const float2*>(buf + k * ROWB + F::piece(col >> 1, k & 7) + (col & 1) * 8); },
+          tid / TI, ck2, t.nyq || kx == 0 ? 1u : 2u, sthr, a.nbins, a.dk, a.volume, wb, wb + PK_MAX_BINS, pk_counts(wb));
+    }
     fence_async_smem();
     __syncwarp();
     if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&done[it % NBUF])) : "memory");
@@ -347,8 +387,9 @@ __global__ void __launch_bounds__(ColWSmem<N, MODE>::T, 1) col_warp(const __grid
   for (int k = group; 2 * seq.pairs + k < seq.count; k += ColW<N>::NG) {
     const ColWTile t = seq.single(k);
     if (MODE == COL_Z_INV_FILTER) weights(t);
-    if (!transform(2 * seq.pairs + k, t)) return;
+    if (!transform(2 * seq.pairs + k, t)) break;
   }
+  if constexpr (PK) pk_finish<SM::T, SM::NW>(wts, a);
 }
 
 }  // namespace es

@@ -1080,7 +1080,7 @@ int es_power_spectrum(es_plan* p, const float* dT, const float* ave, const int* 
   es::PkArgs b;
   static_cast<es::OpArgs&>(b) = base_args(p);
   b.cin = p->T; b.cin_nyq = p->Tnyq;
-  set_maps(b, p, SPEC_T, SPEC_T, true, false);
+  set_maps(b, p, SPEC_T, SPEC_T, true, uses_col_warp(p, false));
   std::memcpy(b.thr, thr, sizeof(int) * nbins);
   b.nbins = nbins; b.dk = p->dk; b.volume = (float)(L * L * L);
   b.pk_out = out;

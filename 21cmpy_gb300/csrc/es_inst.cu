@@ -55,7 +55,7 @@ static cudaError_t launch_col_tma(const OpArgs& base, cudaStream_t s) {
   if (a.col_tile == 1) return launch<col_tma<N, MODE, 1, RS>>(TmaSmem<N, MODE, 1>::bytes, a, ColTile<N, 1>::T, s);
   if (a.col_tile == 2) return launch<col_tma<N, MODE, 2, RS>>(TmaSmem<N, MODE, 2>::bytes, a, ColTile<N, 2>::T, s);
   // tile shape 0 with the large radices is the warp-per-columns form at the sizes that have it
-  if constexpr (ColW<N>::TI > 0 && RS == 0 && MODE != COL_Z_FWD_PK) return cudaErrorInvalidValue;
+  if constexpr (ColW<N>::TI > 0 && RS == 0) return cudaErrorInvalidValue;
   else return launch<col_tma<N, MODE, 0, RS>>(TmaSmem<N, MODE, 0>::bytes, a, ColTile<N, 0>::T, s);
 }
 
@@ -65,8 +65,10 @@ static cudaError_t launch_col(const OpArgs& a, cudaStream_t s) {
   if (a.variant == 0)
     return launch<col_pass<N, MODE>>(ColSmem<N, MODE>::bytes, static_cast<const typename ColArgs<MODE>::type&>(a),
                                      ColCfg<N>::T, s);
-  if constexpr (ColW<N>::TI > 0 && MODE != COL_Z_FWD_PK) {
-    if (a.col_warp) return launch<col_warp<N, MODE>>(ColWSmem<N, MODE>::bytes, a, ColWSmem<N, MODE>::T, s);
+  if constexpr (ColW<N>::TI > 0) {
+    if (a.col_warp)
+      return launch<col_warp<N, MODE>>(ColWSmem<N, MODE>::bytes, static_cast<const typename ColArgs<MODE>::type&>(a),
+                                       ColWSmem<N, MODE>::T, s);
   }
   if constexpr (MODE == COL_Z_INV_FILTER || MODE == COL_Y_INV) {
     if (a.col_radix == 1) return launch_col_tma<N, MODE, 1>(a, s);

@@ -394,14 +394,13 @@ __device__ __forceinline__ unsigned* pk_counts(float* bins) { return reinterpret
 // N/2 / NSEG short steps and one butterfly; the few tiles at small k hold most bins, and set the tail;
 // merging lanes at every bin change of any of them, the earlier way, cost more than the transform
 // (z forward + binning at 256^3: 99 us with 20 bins and 232 us with 100, the pass without binning 21 us;
-// now 45 us and 62 us).  ck2: the column's ky^2 + kx^2; wgt: modes a value stands for.
-template <int N, int TI, int T>
-__device__ __forceinline__ void pk_bin_columns(const float2* g, int ck2, unsigned wgt, const int* thr, int nbins, float dk,
+// then 45 us and 62 us).  ck2: the column's ky^2 + kx^2; wgt: modes a value stands for.
+// at(k): element k of the thread's column, whose |kz| values seg KS + 1 .. seg KS + KS (0 too for seg 0) it takes.
+template <int N, int KS, class At>
+__device__ __forceinline__ void pk_bin_segment(At at, int seg, int ck2, unsigned wgt, const int* thr, int nbins, float dk,
                                                float volume, float* sum_p, float* sum_k, unsigned* count) {
-  constexpr int M = N / 2, NSEG = T / TI, KS = (M + NSEG - 1) / NSEG;
-  static_assert(NSEG * TI == T && T % 32 == 0, "threads must cover whole columns");
+  constexpr int M = N / 2;
   const float inv = 1.0f / (2.0f * 9.8696044010893586f * volume);
-  const int col = threadIdx.x % TI, seg = threadIdx.x / TI;
   int k = seg == 0 ? 0 : seg * KS + 1;
   const int end = min(seg * KS + KS, M);                 // last |kz| of this thread
   if (k == 0 && ck2 == 0) k = 1;                         // the mean (k = 0) is excluded
@@ -422,11 +421,11 @@ __device__ __forceinline__ void pk_bin_columns(const float2* g, int ck2, unsigne
       for (; k <= end; ++k) {
         const int k2 = k * k + ck2;
         if (k2 > top) break;
-        const float2 u = g[k * TI + col];
+        const float2 u = at(k);
         float pw = u.x * u.x + u.y * u.y;
         unsigned n = wgt;
         if (k > 0 && k < M) {
-          const float2 m = g[(N - k) * TI + col];
+          const float2 m = at(N - k);
           pw += m.x * m.x + m.y * m.y;
           n += wgt;
         }
@@ -462,13 +461,23 @@ __device__ __forceinline__ void pk_bin_columns(const float2* g, int ck2, unsigne
   }
 }
 
+// A tile of TI columns by the T threads of a CTA: column threadIdx.x mod TI, in T / TI segments.
+template <int N, int TI, int T>
+__device__ __forceinline__ void pk_bin_columns(const float2* g, int ck2, unsigned wgt, const int* thr, int nbins, float dk,
+                                               float volume, float* sum_p, float* sum_k, unsigned* count) {
+  constexpr int NSEG = T / TI, KS = (N / 2 + NSEG - 1) / NSEG;
+  static_assert(NSEG * TI == T && T % 32 == 0, "threads must cover whole columns");
+  const int col = threadIdx.x % TI, seg = threadIdx.x / TI;
+  pk_bin_segment<N, KS>([&](int k) { return g[k * TI + col]; }, seg, ck2, wgt, thr, nbins, dk, volume, sum_p, sum_k, count);
+}
+
 // Per-CTA bins (fixed warp order) -> partials -> the last CTA of each group of consecutive CTAs adds
 // the group's partials -> the last group adds the groups', each in a fixed order, and writes ps_ave,
 // k_ave and the count (rounded to float32 once, at the end).  About sqrt(grid) CTAs form a group, so
 // either step reads ~20 partials per value, all in flight at once: the single last CTA that read all
 // 304 of them one after the other took 45 us of the 256^3 pass with 20 bins and 160 us with 100.
 constexpr int kPkGroups = 48;                         // arrival counters of the groups, from counter[16]
-template <int T>
+template <int T, int NWB = T / 32>                    // NWB: warps that have bins
 __device__ __forceinline__ void pk_finish(float* bins, const OpArgs& a) {
   __syncthreads();
   const int nb3 = 3 * a.nbins, grid = (int)gridDim.x;
@@ -480,11 +489,11 @@ __device__ __forceinline__ void pk_finish(float* bins, const OpArgs& a) {
     const int q = idx / a.nbins, bin = idx % a.nbins;
     if (q < 2) {
       float s = 0.f;
-      for (int w = 0; w < T / 32; ++w) s += bins[w * PK_MAX_BINS * 3 + q * PK_MAX_BINS + bin];
+      for (int w = 0; w < NWB; ++w) s += bins[w * PK_MAX_BINS * 3 + q * PK_MAX_BINS + bin];
       a.partials[(size_t)blockIdx.x * nb3 + idx] = s;
     } else {
       unsigned s = 0u;
-      for (int w = 0; w < T / 32; ++w) s += pk_counts(bins + w * PK_MAX_BINS * 3)[bin];
+      for (int w = 0; w < NWB; ++w) s += pk_counts(bins + w * PK_MAX_BINS * 3)[bin];
       a.partials[(size_t)blockIdx.x * nb3 + idx] = __uint_as_float(s);
     }
   }
