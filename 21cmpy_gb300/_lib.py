@@ -128,6 +128,8 @@ _PROTOS = {
     "pf_last_error": (C.c_int, [C.c_char_p, C.c_int]),
     "ic_spectrum": (C.c_int, [C.c_int, C.c_float, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int,
                               C.c_void_p, C.c_void_p]),
+    "es_density": (C.c_int, [C.c_void_p, C.c_float, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_void_p,
+                             C.c_float, C.c_void_p, C.c_void_p]),
     "ic_shape": (C.c_int, [C.c_int, C.c_float, C.c_void_p, C.c_int, C.c_int, C.c_float, C.c_int, C.c_void_p,
                            C.c_void_p]),
     "ic_sampled_fields": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_float, C.c_int, C.c_int, C.c_int,
@@ -177,7 +179,7 @@ def last_error(lib=None) -> str:
 
 def check(fn: str, code: int, lib=None):
     if code != ES_OK:
-        if fn[:3] in ("sg_", "pf_", "ic_"):
+        if fn[:3] in ("sg_", "pf_", "ic_") and fn != "ic_sampled_fields":   # the engine reports that one
             lib = lib or load()
             buf = C.create_string_buffer(1024)
             {"sg_": lib.sg_last_error, "pf_": lib.pf_last_error, "ic_": lib.ic_last_error}[fn[:3]](buf, len(buf))

@@ -718,6 +718,9 @@ FftLayout fft_layout(int n, int spectra) {
 // ic.cu: folds the shaped half spectrum of an n^3 field onto h^3 (see ic_sampled_fields)
 __attribute__((visibility("hidden"))) cudaError_t ic_launch_fold(int n, int h, float dk, const float2* half, const float2* nyq, int filter, float R, int ref_compat,
                            int first, int count, float2* const* out, float2* const* out_nyq, cudaStream_t s);
+// ic.cu: ic_spectrum's kernel, writing the plan's layout too (see es_density)
+__attribute__((visibility("hidden"))) cudaError_t ic_launch_spectrum(int n, float box_len, const float* nre, const float* nim, const float* K,
+                               const float* P, int tn, float2* out, float2* main, float2* nyq, cudaStream_t s);
 
 extern "C" {
 
@@ -1154,6 +1157,19 @@ int es_fft_plan_create(int n, double box_len, int spectra, const void* twiddles,
     return cleanup(fail(ES_E_CUDA, "es_fft_plan_create: memset failed"));
   *out = p;
   return ES_OK;
+}
+
+int es_density(es_plan* p, float box_len, const float* normals_re, const float* normals_im, const float* k_table,
+               const float* p_table, int table_n, void* out_half, float scale, float* out, void* stream) {
+  if (!p || !(box_len > 0.f) || !normals_re || !normals_im || !k_table || !p_table || !out_half || !out || table_n < 2)
+    return fail(ES_E_ARG, "es_density: bad arguments");
+  DeviceGuard g(p->device);
+  cudaStream_t s = (cudaStream_t)stream;
+  const int f = fft_spec(p);
+  const cudaError_t e = ic_launch_spectrum(p->n, box_len, normals_re, normals_im, k_table, p_table, table_n, (float2*)out_half,
+                                           p->spec[f], p->spec_nyq[f], s);
+  if (e != cudaSuccess) return fail(ES_E_CUDA, "es_density: launch failed: %s", cudaGetErrorString(e));
+  return inverse_from(p, f, scale, out, s);
 }
 
 int ic_sampled_fields(es_plan* big, const void* half, es_plan* small, int filter_type, float R, int ref_compat, int first,

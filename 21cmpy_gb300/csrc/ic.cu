@@ -58,12 +58,14 @@ struct Quad {
 
 // A warp takes the row quads in turn, the table lies in shared memory (when it fits) and is entered near
 // the right place: 512^3 662 us one element at a time, with a division for its index and a binary search in
-// global memory, 234 us now (1.08 GB moved: 160 us).  Bound by DRAM.
+// global memory, 234 us now (1.08 GB moved: 160 us).  Bound by DRAM.  With `main` it also
+// writes the spectrum in a transform plan's layout, 308 us at 512^3; converting its output there took 203 us more.
 constexpr int kTabMax = 2048;                         // table entries held in shared memory
 __global__ void __launch_bounds__(256) spectrum_kernel(int n, float dk, const float* __restrict__ nre,
                                                        const float* __restrict__ nim, const float* __restrict__ Kg,
                                                        const float* __restrict__ Pg, int tn, float vol,
-                                                       float2* __restrict__ out) {
+                                                       float2* __restrict__ out, float2* __restrict__ main,
+                                                       float2* __restrict__ nyq) {
   __shared__ float tab[2 * kTabMax];
   const bool fits = tn <= kTabMax;
   if (fits)
@@ -111,7 +113,9 @@ __global__ void __launch_bounds__(256) spectrum_kernel(int n, float dk, const fl
             v = make_float2(__fmul_rn(amp, __fmul_rn(__fadd_rn(re[r], nre[mid]), 0.5f)),
                             __fmul_rn(amp, __fmul_rn(__fsub_rn(im[r], nim[mid]), 0.5f)));
           }
-          out[idx] = ksq == 0.0f ? make_float2(0.f, 0.f) : v;
+          if (ksq == 0.0f) v = make_float2(0.f, 0.f);
+          out[idx] = v;
+          if (main) (k2 < n / 2 ? main[(size_t)q.rows[r] * (n / 2) + k2] : nyq[q.rows[r]]) = v;
         }
       }
     }
@@ -328,6 +332,15 @@ __attribute__((visibility("hidden"))) cudaError_t ic_launch_fold(int n, int h, f
   return cudaGetLastError();
 }
 
+// es_engine.cu: the spectrum in numpy's layout and, if main is given, in a transform plan's
+__attribute__((visibility("hidden"))) cudaError_t ic_launch_spectrum(int n, float box_len, const float* nre, const float* nim, const float* K,
+                               const float* P, int tn, float2* out, float2* main, float2* nyq, cudaStream_t s) {
+  const float dk = (float)(2.0 * M_PI / (double)box_len);
+  const float vol = box_len * box_len * box_len;
+  ic::spectrum_kernel<<<grid_for((long)n * n * (n / 2 + 1)), 256, 0, s>>>(n, dk, nre, nim, K, P, tn, vol, out, main, nyq);
+  return cudaGetLastError();
+}
+
 extern "C" {
 
 int ic_spectrum(int n, float box_len, const float* normals_re, const float* normals_im, const float* k_table,
@@ -335,12 +348,8 @@ int ic_spectrum(int n, float box_len, const float* normals_re, const float* norm
   if (n < 2 || n > 2048 || !(box_len > 0.f) || !normals_re || !normals_im || !k_table || !p_table || !out_half ||
       table_n < 2)
     return icfail(ES_E_ARG, "ic_spectrum: bad arguments");
-  const float dk = (float)(2.0 * M_PI / (double)box_len);
-  const float vol = box_len * box_len * box_len;
-  const long total = (long)n * n * (n / 2 + 1);
-  ic::spectrum_kernel<<<grid_for(total), 256, 0, (cudaStream_t)stream>>>(
-      n, dk, normals_re, normals_im, k_table, p_table, table_n, vol, (float2*)out_half);
-  const cudaError_t e = cudaGetLastError();
+  const cudaError_t e = ic_launch_spectrum(n, box_len, normals_re, normals_im, k_table, p_table, table_n, (float2*)out_half,
+                                           nullptr, nullptr, (cudaStream_t)stream);
   return e == cudaSuccess ? ES_OK : icfail(ES_E_CUDA, "ic_spectrum launch: %s", cudaGetErrorString(e));
 }
 

@@ -87,6 +87,17 @@ class InitialConditions:
         _lib.check("ic_spectrum", rc, self.lib)
         return out
 
+    def _density(self, nre: torch.Tensor, nim: torch.Tensor):
+        """``spectrum`` and its inverse transform times ``norm``, in one call."""
+        n = self.dim
+        H = torch.empty((n, n, n // 2 + 1), dtype=torch.complex64, device=self.device)
+        box = torch.empty((n, n, n), dtype=torch.float32, device=self.device)
+        nre, nim = nre.contiguous(), nim.contiguous()
+        rc = self.lib.es_density(self._fft.handle, C.c_float(self.box_len), _p(nre), _p(nim), _p(self.K), _p(self.P),
+                                 TABLE_N, _p(H), C.c_float(float(np.float32(self.norm))), _p(box), self._fft._on(None))
+        _lib.check("es_density", rc, self.lib)
+        return H, box
+
     def shaped(self, H: torch.Tensor, component: int, filter_type: int = 0, ref_compat: bool = False) -> torch.Tensor:
         out = torch.empty_like(H)
         rc = self.lib.ic_shape(self.dim, C.c_float(self.box_len), _p(H), int(component), int(filter_type),
@@ -107,9 +118,8 @@ class InitialConditions:
         """{"deltax": DIM^3 density at z = 0, "smoothed": HII_DIM^3 smoothed density,
         "vx", "vy", "vz": HII_DIM^3 displacement per unit growth (initialize.py:83-109)}."""
         nre, nim = self.normals(seed) if normals is None else normals
-        H = self.spectrum(nre, nim)
-        out = {"spectrum": H}
-        out["deltax"] = self._fft.fft_c2r(H, scale=self.norm)
+        H, deltax = self._density(nre, nim)
+        out = {"spectrum": H, "deltax": deltax}
         names = ("smoothed", "vx", "vy", "vz")
         if self._small is not None:
             out.update(zip(names, self._sampled(H, -1, 4, self.norm, filter_type, ref_compat)))

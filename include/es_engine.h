@@ -322,6 +322,10 @@ int pf_last_error(char* buf, int len);
  * ic_subsample replaces subsample (initialize.cu:133-146): small = large[floor(a pf + 0.5)] * scale. */
 int ic_spectrum(int n, float box_len, const float* normals_re, const float* normals_im, const float* k_table,
                 const float* p_table, int table_n, void* out_half, void* stream);
+/* ic_spectrum of the plan's size and its inverse transform times scale (out: device float n^3) in one call:
+ * the same values as ic_spectrum and es_fft_c2r_scaled. */
+int es_density(es_plan* plan, float box_len, const float* normals_re, const float* normals_im, const float* k_table,
+               const float* p_table, int table_n, void* out_half, float scale, float* out, void* stream);
 int ic_shape(int n, float box_len, const void* in_half, int component, int filter_type, float R, int ref_compat,
              void* out_half, void* stream);
 /* The boxes that ic_shape, the inverse transform and ic_subsample make of a DIM^3 field's half spectrum
