@@ -83,7 +83,12 @@ static cudaError_t launch_r2c(const OpArgs& a, cudaStream_t s) {
     case 1: return launch<row2_r2c<N, PRO, 1>>(Row2Smem<N, false, 1>::bytes, a, RowTile<N, 1>::T, s);
     case 2: return launch<row2_r2c<N, PRO, 2>>(Row2Smem<N, false, 2>::bytes, a, RowTile<N, 2>::T, s);
     case 3: return launch<row2_r2c<N, PRO, 3>>(Row2Smem<N, false, 3>::bytes, a, RowTile<N, 3>::T, s);
-    default: return launch<row2_r2c<N, PRO, 0>>(Row2Smem<N, false, 0>::bytes, a, RowTile<N, 0>::T, s);
+    default:
+      // tile shape 0 is the warp-per-rows form at the sizes that have it
+      if constexpr (RowWF<N>::ON)
+        return launch<row_warp_r2c<N, PRO>>(RowWF<N>::bytes, a, RowWCfg<N>::T, s);
+      else
+        return launch<row2_r2c<N, PRO, 0>>(Row2Smem<N, false, 0>::bytes, a, RowTile<N, 0>::T, s);
   }
 }
 

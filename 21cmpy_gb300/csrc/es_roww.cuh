@@ -13,6 +13,7 @@
 //
 // What bounds it: instruction issue (the erfc sum is half of it).  The older form (es_rows.cuh) spent
 // 1018 warp instructions per tile and warp at 256^3, with four CTA barriers a tile (issue active 60 %).
+// 256^3: 46.5 -> 38.8 us; 512^3: 395 -> 260 us, 1.6 GB at 0.91 of the copy rate.
 // Thread for thread, the last stage, the running sums and the grid are the older form's, so the
 // grid-wide sums come out the same bit for bit.
 #pragma once
@@ -76,6 +77,34 @@ __device__ __forceinline__ bool grid_sum_as(float mine, float* partials, unsigne
   if (threadIdx.x == 0) *counter = 0u;
   *total = s;
   return true;
+}
+
+// First-stage butterfly of a lane (h: its half where two lanes share one).
+template <class C, bool INV> __device__ __forceinline__ void row_first_dft(float2* v, int h) {
+  if constexpr (C::HALF) {
+    // radix 16 over two lanes: each takes the radix-8 DFT of the even or the odd samples, the odd
+    // ones are turned by w_16^k, and the halves are combined across the pair (Dft<16>)
+    static_assert(C::R0 == 16, "half butterflies are radix 8");
+    constexpr float c1 = 0.92387953251128674f, s1 = 0.38268343236508978f, rt = 0.70710678118654752f;
+    Dft<8, INV>::run(v);
+    if (h) {
+      v[1] = twid<INV>(v[1], c1, -s1);
+      v[2] = twid<INV>(v[2], rt, -rt);
+      v[3] = twid<INV>(v[3], s1, -c1);
+      v[4] = rot<INV>(v[4]);
+      v[5] = twid<INV>(v[5], -s1, -c1);
+      v[6] = twid<INV>(v[6], -rt, -rt);
+      v[7] = twid<INV>(v[7], -c1, -s1);
+    }
+    const float sg = h ? -1.0f : 1.0f;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {                      // even lane: e + o; odd lane: e - o (outputs 8 + k)
+      const float ox = __shfl_xor_sync(0xffffffffu, v[k].x, 1), oy = __shfl_xor_sync(0xffffffffu, v[k].y, 1);
+      v[k] = make_float2(fmaf(v[k].x, sg, ox), fmaf(v[k].y, sg, oy));
+    }
+  } else {
+    Dft<C::R0, INV>::run(v);
+  }
 }
 
 template <int N, int EPI>
@@ -180,30 +209,7 @@ __global__ void __launch_bounds__(RowWCfg<N>::T, RowOcc<N, 0>::MINB) row_warp_c2
       for (int q = 0; q < RW * M / 16; q += 32)
         if (q + lane < RW * M / 16) l2_discard(g + 16 * q);
     }
-    if constexpr (HALF) {
-      // radix 16 over two lanes: each takes the radix-8 DFT of the even or the odd samples, the odd
-      // ones are turned by w_16^k, and the halves are combined across the pair (Dft<16>)
-      static_assert(R0 == 16, "half butterflies are radix 8");
-      constexpr float c1 = 0.92387953251128674f, s1 = 0.38268343236508978f, rt = 0.70710678118654752f;
-      Dft<8, true>::run(v);
-      if (h) {
-        v[1] = twid<true>(v[1], c1, -s1);
-        v[2] = twid<true>(v[2], rt, -rt);
-        v[3] = twid<true>(v[3], s1, -c1);
-        v[4] = rot<true>(v[4]);
-        v[5] = twid<true>(v[5], -s1, -c1);
-        v[6] = twid<true>(v[6], -rt, -rt);
-        v[7] = twid<true>(v[7], -c1, -s1);
-      }
-      const float sg = h ? -1.0f : 1.0f;
-#pragma unroll
-      for (int k = 0; k < 8; ++k) {                      // even lane: e + o; odd lane: e - o (outputs 8 + k)
-        const float ox = __shfl_xor_sync(0xffffffffu, v[k].x, 1), oy = __shfl_xor_sync(0xffffffffu, v[k].y, 1);
-        v[k] = make_float2(fmaf(v[k].x, sg, ox), fmaf(v[k].y, sg, oy));
-      }
-    } else {
-      Dft<R0, true>::run(v);
-    }
+    row_first_dft<C, true>(v, h);
     __syncwarp();                                        // every lane has read its rows
     // exchange: output r of butterfly j0 goes to slot j0 R0 + (r ^ j0)
     {
@@ -306,6 +312,152 @@ __global__ void __launch_bounds__(RowWCfg<N>::T, RowOcc<N, 0>::MINB) row_warp_c2
       a.stats_out[1] = mean;
       a.stats_out[2] = a.normalize ? a.fc_mean / mean : 1.f;
     }
+  }
+}
+
+// Row R2C pass in the same form: real rows -> half-spectrum rows (slot 0 holds (X[0], X[N/2])), with a scale
+// or P(k) prologue.  The rows stay in one of the warp's NB buffers from their arrival to their stores: first
+// stage out of it and back into it, last stage likewise in natural order, then the split by pairs (t, M - t)
+// straight to global memory.  Arithmetic as row2_r2c, whose values pass through shared memory after the
+// prologue: the scaling is kept out of the first butterfly's multiply-adds.
+// 512^3: 235 -> 176 us, 1.07 GB at 0.90 of the copy rate, and so bound by DRAM.  256^3 keeps the older form:
+// the pass alone takes 24 us against 27 us here, but a box 2746 us against 2736 and its products 160 against
+// 156, with both neighbours overlapping the pass; at 128^3 there is nothing between them (911 us a box).
+template <int N> struct RowWF {
+  static constexpr bool ON = RowW<N>::NP > 0 && N >= 512;
+  static constexpr int NB = 3;
+  using C = RowWCfg<N>;
+  static constexpr int TAB = (N / 4 + 1) + C::TW;        // split and last-stage twiddles
+  static constexpr int BARS = (TAB * 8 + 15) / 16 * 16, BUFS = (BARS + C::NW * 32 + 127) / 128 * 128;
+  static constexpr int bytes = BUFS + C::NW * NB * C::XBUF + 128;
+};
+
+template <int N, int PRO>
+__global__ void __launch_bounds__(RowWCfg<N>::T) row_warp_r2c(const __grid_constant__ OpArgs a) {
+  using C = RowWCfg<N>;
+  using F = RowWF<N>;
+  constexpr int M = C::M, RL = C::RL, RW = C::RW, R0 = C::R0, R1 = C::R1, NSL = C::NSL, NB = F::NB, PITCH = C::PITCH;
+  constexpr bool HALF = C::HALF;
+  constexpr int J0 = R1, V0 = HALF ? R0 / 2 : R0;
+  static_assert(NB <= 4 && RW * (M / 2) % 32 == 0, "four mbarriers a warp; whole rounds of pairs");
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  unsigned char* base = align_smem<128>(smem_raw);
+  float2* wsp = reinterpret_cast<float2*>(base);         // w_N^t, t <= M/2
+  float2* tws = wsp + M / 2 + 1;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(base + F::BARS) + 4 * warp;
+  unsigned char* bufs = base + F::BUFS + warp * NB * C::XBUF;
+
+  constexpr int ntiles = N * N / RL;
+  const int my_count = (int)blockIdx.x < ntiles ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+  auto pair_at = [&](int it) { return ((blockIdx.x + it * gridDim.x) * RL + warp * RW) * M; };
+  auto issue = [&](int it) {
+    const uint64_t pol = l2_policy(a.hint_in);
+    uint64_t* bar = &bars[it % NB];
+    unsigned char* dst = bufs + (it % NB) * C::XBUF;
+    const float2* src = a.rin + pair_at(it);
+    mbar_expect_tx(bar, (uint32_t)(RW * M * 8) + stall_bytes(a.stall, it));
+    if (PITCH == M) {
+      bulk_load(dst, src, RW * M * 8, bar, pol);
+    } else {
+#pragma unroll
+      for (int l = 0; l < RW; ++l) bulk_load(dst + l * PITCH * 8, src + l * M, M * 8, bar, pol);
+    }
+  };
+  if (lane == 0) {
+    for (int b = 0; b < NB; ++b) mbar_init(&bars[b], 1);
+    fence_mbar_init();
+    fence_async_smem();
+  }
+  for (int i = threadIdx.x; i <= M / 2; i += C::T) wsp[i] = a.tw[i];
+  for (int i = threadIdx.x; i < C::TW; i += C::T) tws[i] = a.tw[(i % NSL) * (i / NSL + 1) * 2];
+  pdl_wait();
+  if (lane == 0)
+    for (int it = 0; it < NB && it < my_count; ++it) issue(it);
+  pdl_trigger();
+  float sc = a.scale, sh = 0.f;
+  if (PRO == PRO_PK) {
+    const float ave = *a.ave;
+    // g = (x / ave - 1) V / N^3  (delta_T.py:80-82), optionally times ave
+    sc = a.pk_norm / ave;
+    sh = -a.pk_norm;
+    if (a.dimensional) { sc *= ave; sh *= ave; }
+  }
+  __syncthreads();
+
+  const int l0 = HALF ? lane / (2 * J0) : lane / J0, j0 = HALF ? (lane >> 1) % J0 : lane % J0, h = HALF ? lane & 1 : 0;
+  const int l = lane / NSL, j = lane % NSL;
+  for (int it = 0; it < my_count; ++it) {
+    float2* X = reinterpret_cast<float2*>(bufs + (it % NB) * C::XBUF);
+    const uint32_t pair0 = pair_at(it);
+    if (!__all_sync(0xffffffffu, mbar_wait(&bars[it % NB], (uint32_t)((it / NB) & 1), a.wait_log2))) {
+      // a wait ran out: record it; the copies in flight land (bounded waits) before the warp leaves
+      if (lane == 0) {
+        atomicOr(a.err, ES_DEV_ERR_TIMEOUT);
+        for (int q = it; q < it + NB && q < my_count; ++q) mbar_wait(&bars[q % NB], (uint32_t)((q / NB) & 1), a.wait_log2);
+      }
+      __syncwarp();
+      break;
+    }
+    float2 v[V0];
+    {
+      const float2* x = X + l0 * PITCH + j0 + h * (M / R0);
+#pragma unroll
+      for (int k = 0; k < V0; ++k) {
+        const float2 r = x[k * (HALF ? 2 : 1) * (M / R0)];
+        v[k] = PRO == PRO_PK ? make_float2(fmaf(r.x, sc, sh), fmaf(r.y, sc, sh))
+                             : make_float2(__fmul_rn(r.x, sc), __fmul_rn(r.y, sc));
+      }
+    }
+    row_first_dft<C, false>(v, h);
+    __syncwarp();                                        // every lane has read its rows
+    {
+      float2* x = X + l0 * PITCH + j0 * R0 + h * V0;
+#pragma unroll
+      for (int k = 0; k < V0; ++k) x[k ^ (HALF ? (j0 & 7) : j0)] = v[k];
+    }
+    __syncwarp();
+    float2 z[R1];
+    {
+      const float2* x = X + l * PITCH;
+#pragma unroll
+      for (int r = 0; r < R1; ++r) z[r] = x[r * R0 + (j ^ r)];
+    }
+#pragma unroll
+    for (int r = 1; r < R1; ++r) {
+      const float2 w = tws[(r - 1) * NSL + j];
+      z[r] = twid<false>(z[r], w.x, w.y);
+    }
+    Dft<R1, false>::run(z);
+    __syncwarp();
+#pragma unroll
+    for (int r = 0; r < R1; ++r) X[l * PITCH + j + r * NSL] = z[r];
+    __syncwarp();
+    // X[m] = (Z[m] + conj Z[M-m]) / 2 - i w^m (Z[m] - conj Z[M-m]) / 2 by pairs (t, M - t); item 0 the packed
+    // (X[0], X[N/2]) and the self-paired X[M/2]; w^(M-t) = -conj w^t
+#pragma unroll 4
+    for (int q = lane; q < RW * (M / 2); q += 32) {
+      const int t = q % (M / 2), row = q / (M / 2);
+      const float2* Z = X + row * PITCH;
+      float2* out = a.cout + pair0 + row * M;
+      if (t == 0) {
+        const float2 z0 = Z[0];
+        out[0] = make_float2(z0.x + z0.y, z0.x - z0.y);
+        const float2 zh = Z[M / 2];
+        const float2 th = cmul(wsp[M / 2], make_float2(0.f, zh.y + zh.y));
+        out[M / 2] = make_float2(0.5f * (zh.x + zh.x + th.y), -0.5f * th.x);
+      } else {
+        const int m2 = M - t;
+        const float2 zm = Z[t], zc = Z[m2], w = wsp[t];
+        const float2 t1 = cmul(w, make_float2(zm.x - zc.x, zm.y + zc.y));
+        out[t] = make_float2(0.5f * (zm.x + zc.x + t1.y), 0.5f * (zm.y - zc.y - t1.x));
+        const float2 t2 = cmul(make_float2(-w.x, w.y), make_float2(zc.x - zm.x, zc.y + zm.y));
+        out[m2] = make_float2(0.5f * (zc.x + zm.x + t2.y), 0.5f * (zc.y - zm.y - t2.x));
+      }
+    }
+    fence_async_smem();
+    __syncwarp();
+    if (lane == 0 && it + NB < my_count) issue(it + NB);
   }
 }
 
