@@ -8,7 +8,8 @@
 // with 16 warps per SM, and spends as long at barriers and waiting for its copies as issuing (issue
 // active 47 % in the z inverse, 37 % in the y inverse at 256^3).  Here warps drift apart, so one
 // warp's loads and shared-memory trips hide behind the others' arithmetic, and up to 192 KB of tiles
-// are in flight per SM.  The arithmetic is the same operation for operation.
+// are in flight per SM.  The arithmetic is the same operation for operation.  z inverse + filter / y inverse:
+// 256^3 30.8 / 24.0 -> 23.1 / 16.9 us, 512^3 245 / 233 -> 205 / 186 us (DRAM).
 #pragma once
 #include "es_tma.cuh"
 

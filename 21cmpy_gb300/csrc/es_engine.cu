@@ -551,8 +551,8 @@ es::OpArgs base_args(const es_plan* p) {
 }
 
 // Whether a column pass runs in the warp-per-columns form: sizes that have it, with the default tile
-// shape and radix schedule.  256^3 alone: z inverse + filter 30.9 -> 24.8 us, y inverse 23.8 -> 17.3 us;
-// 512^3: 245 -> 203 us and 233 -> 198 us.
+// shape and radix schedule.  256^3 alone: z inverse + filter 30.9 -> 23.1 us, y inverse 23.8 -> 16.9 us;
+// 512^3: 245 -> 205 us and 233 -> 186 us.
 bool uses_col_warp(const es_plan* p, bool per_radius) {
   return p->col_variant == 1 && p->col_tile == 0 && p->geo.colw_ti > 0 && !(per_radius && p->col_radix);
 }
@@ -724,7 +724,7 @@ __attribute__((visibility("hidden"))) cudaError_t ic_launch_spectrum(int n, floa
 
 extern "C" {
 
-int es_version(void) { return 3; }
+int es_version(void) { return 4; }
 
 int es_last_error(char* buf, int len) {
   if (!buf || len <= 0) return ES_E_ARG;

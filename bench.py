@@ -678,7 +678,7 @@ def run_perturb(dev, hbm_gbs: float, reps: int = 20):
             "l2": "flushed (256 MiB write) before every timed launch",
             "velocities_ms": vel_ms,
             "velocities_workload": "updated velocity boxes at z = 8 from the 512^3 density: forward 512^3 FFT, "
-                                   "3 x (k-space shape, inverse 512^3 FFT, subsample to 128^3)",
+                                   "its shaped spectrum folded to 128^3, 3 inverse 128^3 FFTs",
             "cpu_baseline": {"value": cpu_rate, "unit": "cells/s", "cores": 1, "kind": "port",
                              "sample": f"64 of 512 DIM planes, numpy float32 oracle, one thread, {cpu_s:.1f} s"}}
 
@@ -700,7 +700,7 @@ def run_initial(dev, reps: int = 5):
         e1.synchronize()
     ms = e0.elapsed_time(e1) / reps
     return {"workload": "initial conditions DIM=512, HII_DIM=128, BOX_LEN=128 Mpc: density, smoothed density, "
-                        "3 displacement boxes (5 inverse 512^3 FFTs), normals resident", "ms": ms}
+                        "3 displacement boxes (one inverse 512^3 FFT, 4 of the folded 128^3 spectra), normals resident", "ms": ms}
 
 
 def run_surrogate(dev, reps: int = 20):

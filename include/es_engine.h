@@ -166,7 +166,7 @@ int es_fft_c2r_scaled(es_plan* plan, const void* in_half, float scale, float* ou
  * es_fft_plan_bytes(n, spectra) bytes; it must outlive the plan) with `spectra` (1..4) spectra in it,
  * and the table twiddles[m] = exp(-2 pi i m / n), m < n (device complex64).  Creating it launches one
  * memset on the stream and allocates nothing on the device.  It serves es_fft_r2c, es_fft_c2r(_scaled),
- * es_fft_forward, ic_sampled_fields, the options, es_plan_check and es_plan_destroy; es_forward,
+ * es_fft_forward, es_density, ic_sampled_fields, the options, es_plan_check and es_plan_destroy; es_forward,
  * es_ionize, es_delta_T, es_power_spectrum and es_profile_enable return ES_E_UNSUPPORTED. */
 size_t es_fft_plan_bytes(int n, int spectra);
 int es_fft_plan_create(int n, double box_len, int spectra, const void* twiddles, void* workspace, size_t bytes,
