@@ -155,12 +155,12 @@ __global__ void shape_kernel(int n, float dk, const float2* __restrict__ in, int
 // conj(H[-k0, -k1, n - kz]) of the stored one.  A CTA makes the rows (+-k0', +-k1') of F for every
 // component: GR groups of h/2 + 1 threads, one kz' per thread, share the p^2 aliases, an alias's window
 // and 1 / k^2 serve its four sign combinations, and each element of H is read once for all components.
-// 512^3 -> 128^3, four components: 288 us (0.54 GB read: 80 us; bound by latency, 70 registers), 502 us with the window evaluated for each
-// element; the route through ic_shape, the 512^3 inverse and ic_subsample took 1.2 ms a component.
+// 512^3 -> 128^3, four components: 247 us (0.54 GB read: 80 us; bound by latency: 285 us at 70 registers and
+// three groups, 455 with the next alias' loads ahead at 90), 502 us with the window evaluated for each element; the route through ic_shape, the 512^3 inverse and ic_subsample took 1.2 ms a component.
 // nyq: null for the numpy layout, else H's Nyquist plane apart.
 struct FoldOut { float2 *main[4], *nyq[4]; };
 template <int NC>
-__global__ void __launch_bounds__(544) fold_kernel(int n, int h, float dk, const float2* __restrict__ H,
+__global__ void __launch_bounds__(544, 2) fold_kernel(int n, int h, float dk, const float2* __restrict__ H,
                                                    const float2* __restrict__ nyq, int filter, float R, int k2cut,
                                                    int ref_compat, int first, int groups, FoldOut o) {
   extern __shared__ float2 part[];                      // [groups][4][NC][h/2 + 1]
@@ -308,10 +308,12 @@ static int tophat_cut(float dk, int filter_type, float R, int ref_compat) {
 __attribute__((visibility("hidden"))) cudaError_t ic_launch_fold(int n, int h, float dk, const float2* half, const float2* nyq, int filter, float R, int ref_compat,
                            int first, int count, float2* const* out, float2* const* out_nyq, cudaStream_t s) {
   const int w = h / 2 + 1;
-  int groups = 256 / w;                                 // about 256 threads; at least one group, at most the alias rows
-  const int p2 = (n / h) * (n / h);
-  if (groups > p2) groups = p2;
-  if (groups < 1) groups = 1;
+  // up to 288 threads, and of those the fewest groups that take the alias rows in as many rounds: at
+  // 512 -> 128 four groups take 16 rows in 4 (three in 6: 266 us against 285).  Rows of more than 96 values keep
+  // to 256 threads: their few aliases (p = 2) are better added up by one group, error against float64 2.22e-7
+  // of a 512 -> 256 velocity box against 2.27e-7 by two
+  const int p2 = (n / h) * (n / h), fit = (w <= 96 ? 288 : 256) / w, most = fit < 1 ? 1 : (fit > p2 ? p2 : fit);
+  const int rounds = (p2 + most - 1) / most, groups = (p2 + rounds - 1) / rounds;
   const int threads = (groups * w + 31) / 32 * 32;
   const size_t smem = groups > 1 ? (size_t)groups * 4 * count * w * sizeof(float2) : 0;   // at most 36 KB
   const int cut = tophat_cut(dk, filter, R, ref_compat);
