@@ -188,7 +188,6 @@ __global__ void __launch_bounds__(256) move_cells_kernel(int sw, int parts, cons
   // sums [axis 0][axis 1][axis 2], 0: total, 1: A's share; hi and lo parts
   int hi[2][2][2] = {}, lo[2][2][2] = {};
   if (ok) {
-    float most = 0.0f;
     int m2[P];
 #pragma unroll
     for (int k = 0; k < P; ++k) m2[k] = (b2 >> k) & 1u ? 0 : -1;
@@ -201,7 +200,7 @@ __global__ void __launch_bounds__(256) move_cells_kernel(int sw, int parts, cons
 #pragma unroll
         for (int k = 0; k < P; ++k) {
           const float mass = __fadd_rn(1.0f, __fmul_rn(g0, r.v[k]));
-          most = fabsf(mass) <= most ? most : fabsf(mass);            // NaN stays
+          ok = ok && fabsf(mass) < kLimit;                           // false for NaN, and then for good
           const float up = __fadd_rn(mass, 192.0f);
           const float low = __fsub_rn(mass, __fsub_rn(up, 192.0f));
           const int qh = __float_as_int(up) - 0x43400000, ql = __float_as_int(fmaf(low, kFix, 12582912.0f)) - 0x4B400000;
@@ -225,7 +224,6 @@ __global__ void __launch_bounds__(256) move_cells_kernel(int sw, int parts, cons
           lo[1][i][j] += pl[i][j] & m0;
         }
     }
-    ok = most < kLimit;
   }
   if (!ok) {
     for (int k0 = 0; k0 < planes; ++k0)
