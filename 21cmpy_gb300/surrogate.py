@@ -17,6 +17,7 @@ from __future__ import annotations
 
 import ctypes as C
 import math
+import threading
 from dataclasses import dataclass
 
 import numpy as np
@@ -149,24 +150,50 @@ class SurrogateNet:
         return dws, dbs
 
 
-_smooth_plans = {}
+class _SmoothPlan:
+    """A transform plan that every call for one box size and device shares, with what keeps the calls apart:
+    the spectrum stays in the plan between its two steps."""
+
+    def __init__(self, n: int, device):
+        from .engine import ExcursionSetPlan
+        self.plan = ExcursionSetPlan(n, float(n), max_radii=1, device=device)     # lengths in cells
+        self.lock = threading.Lock()
+        self.done = torch.cuda.Event()
+        self.stream = None               # where the last call was queued, `done` after it
+
+
+_smooth_plans: dict = {}
+_smooth_lock = threading.Lock()
 
 
 def smoothed_fields(delta: torch.Tensor, radii_cells) -> torch.Tensor:
     """The density smoothed with the real-space top hat W(kR) at each radius (in cells): one forward
     transform, then per radius the window and an inverse transform (``es_smooth``).
-    Returns float32 [len(radii), n, n, n]."""
-    from .engine import ExcursionSetPlan
+    Returns float32 [len(radii), n, n, n].
+
+    Calls from several threads and streams are kept in order.  A call captured in a graph uses the same plan,
+    and its replays are for the caller to order against other calls."""
     n = delta.shape[0]
     key = (n, str(delta.device))
-    if key not in _smooth_plans:
-        _smooth_plans[key] = ExcursionSetPlan(n, float(n), max_radii=1, device=delta.device)   # lengths in cells
-    plan = _smooth_plans[key]
+    with _smooth_lock:
+        if key not in _smooth_plans:
+            _smooth_plans[key] = _SmoothPlan(n, delta.device)
+        shared = _smooth_plans[key]
+    plan = shared.plan
     out = torch.empty((len(radii_cells), n, n, n), dtype=torch.float32, device=delta.device)
     radii = (C.c_float * len(radii_cells))(*[float(R) for R in radii_cells])
-    with torch.cuda.device(delta.device):
-        plan.forward(delta)
-        _lib.check("es_smooth", plan.lib.es_smooth(plan.handle, radii, len(radii_cells), _p(out), _stream()), plan.lib)
+    with torch.cuda.device(delta.device), shared.lock:
+        stream = torch.cuda.current_stream()
+        capturing = torch.cuda.is_current_stream_capturing()
+        if not capturing and shared.stream is not None and shared.stream != stream:
+            stream.wait_event(shared.done)
+        try:
+            plan.forward(delta)
+            _lib.check("es_smooth", plan.lib.es_smooth(plan.handle, radii, len(radii_cells), _p(out), _stream()), plan.lib)
+        finally:
+            if not capturing:
+                shared.done.record(stream)
+                shared.stream = stream
     return out
 
 
