@@ -262,18 +262,115 @@ __global__ void __launch_bounds__(T) delta_T_kernel(const float2* xH, const floa
 //    centre on each side counts.  Eight lanes share a word, each taking every eighth (dz, dy), and
 //    OR-reduce; words that are full already are left.  The work is N^3 / 32 x pi r^2 short steps
 //    whatever the number of centres.
-//  * One warp per centre (few centres): the warp paints the ball of each centre it finds in its
-//    part of the bitmap, row by row with atomic ORs: work ~ centres x (2 r + 1)^2 / 32 row steps.
+//  * Ball by ball (few centres): a CTA lists the centres in its part of the bitmap, and its threads OR
+//    the rows of their balls, one row each: work ~ centres x (2 r + 1)^2 rows.
 //
-// A step of the first kind costs about a third of one of the second and is shared by 32 cells, so by
-// work alone the lines cross near one centre in 1000 cells; but centres come in clusters, which keep
-// a few warps busy, and at one in 1024 the second way took 62 us at 96^3 (radius 7 cells) where the
-// first takes 22 us.  Below one in 4096 it takes 13 us or less against the first's 28 us.
+// By work alone the lines cross where a centre's rows cost as much as the words of as many cells: one centre
+// in 50 cells at 512^3, and no lower in small boxes, where both ways are bound by latency.  Measured on either side
+// of one in 64, balls (radius in cells, cells per centre) against dilation:
+//   512^3: (6.8, 74) 2304 / 3177 us, (5.1, 83) 1481 / 2245, (5.6, 44) 2642 / 2504, (3.5, 43) 1117 / 1116;
+//   256^3: (6.6, 80) 307 / 385, (2.6, 81) 51 / 92, (5.4, 55) 322 / 300, (1.5, 34) 43 / 74;
+//   128^3: (2.6, 80) 16 / 18, (2.2, 55) 18 / 18;  96^3: (2.6, 76) 12 / 12, (2.2, 55) 14 / 12.
+// Far from it: 512^3 (15.9, 80805) 57 / 12133, (10.8, 1320) 444 / 5968; 96^3 (8.3, 6) 403 / 61.
+// Centres come in clusters: with one warp for the centres of a word most warps had none (256^3 (17, 3404)
+// 524 us against 106; a list of all centres dealt to the warps in turn: 102).
 // 96^3, 30 radii, z = 8: painting every centre's ball took 196 us a radius (the words of a dense region are
 // ORed ~1000 times), this less than 20 us (10 us at z = 10); the row pass, which used to append the centres to a list through one
-// counter, went from 14.7 to 10.0 us.  Bound by the latency of the loads and of the launch.
+// counter, went from 14.7 to 10.0 us.  Bound by the latency of the loads and of the launch in small boxes, by issue in large ones.
 constexpr int kPaintTab = 2048;       // (dz, dy, w) entries of the ball held in shared memory at a time
-constexpr int kPaintSparse = 4096;    // cells per centre from which the warp-per-centre way is taken
+constexpr int kPaintSparse = 64;      // cells per centre above which the ball-by-ball way is taken
+constexpr int kPaintList = 1024;      // of which a list of centres takes this many (a thread may bring 128)
+
+// Entries e0 .. e0 + count - 1 of the ball's (dz, dy) square, packed with the half-width w (all ones: outside the ball).
+__device__ __forceinline__ void ball_rows(uint32_t* tab, int e0, int count, int rr, int r2max) {
+  const int side = 2 * rr + 1;
+  for (int e = threadIdx.x; e < count; e += blockDim.x) {
+    const int dz = (e0 + e) / side - rr, dy = (e0 + e) % side - rr;
+    const int rem = r2max - dz * dz - dy * dy;
+    tab[e] = rem < 0 ? 0xffffffffu
+                     : ((uint32_t)(dz + 1023) << 21) | ((uint32_t)(dy + 1023) << 10) | (uint32_t)min(es::isqrt_dev(rem), 1023);
+  }
+}
+
+// The second way.  Words are dealt to the CTAs in turn (by four, which a thread reads at once, where there are
+// more than the grid's threads), so that a cluster of centres is shared by many; a CTA lists the centres in its
+// words, and its threads take the rows of all their balls evenly.  tab (kPaintTab entries): rows of the ball,
+// made once where they fit and only if the CTA has a centre, then the list.
+__device__ __forceinline__ void paint_centres(uint32_t* tab, int rr, int r2max, const uint32_t* __restrict__ centres,
+                                              uint32_t* flags, int n, int nw, uint32_t last_mask, int periodic) {
+  constexpr int kRows = kPaintTab - kPaintList;
+  uint32_t* list = tab + kRows;                          // z, y, x
+  __shared__ int taken, listed;
+  const uint32_t words = (uint32_t)n * n * nw;
+  const bool four = words > gridDim.x * blockDim.x && nw % 4 == 0;     // of one row
+  const uint32_t groups = four ? words / 4 : words;
+  const int side2 = (2 * rr + 1) * (2 * rr + 1);
+  const bool one_tab = side2 <= kRows;
+  bool have_tab = false;
+  if (threadIdx.x == 0) taken = listed = 0;
+  for (uint32_t g0 = blockIdx.x; g0 < groups; g0 += blockDim.x * gridDim.x) {     // uniform over the CTA
+    const uint32_t g = g0 + threadIdx.x * gridDim.x;
+    uint32_t w[4] = {0u, 0u, 0u, 0u}, at = 0u;
+    if (g < groups) {
+      const uint32_t i = four ? 4u * g : g, row = i / (uint32_t)nw, t = i % (uint32_t)nw;
+      if (four) {
+        const uint4 u = reinterpret_cast<const uint4*>(centres)[g];
+        w[0] = u.x; w[1] = u.y; w[2] = u.z; w[3] = u.w;
+        if ((int)t == nw - 4) w[3] &= last_mask;
+      } else {
+        w[0] = centres[i] & ((int)t == nw - 1 ? last_mask : 0xffffffffu);
+      }
+      at = ((row / (uint32_t)n) << 20) | ((row % (uint32_t)n) << 10) | (32u * t);
+    }
+    int left = __syncthreads_or((w[0] | w[1] | w[2] | w[3]) != 0u);
+    while (left) {
+      const int k = __popc(w[0]) + __popc(w[1]) + __popc(w[2]) + __popc(w[3]);
+      if (k) {
+        int pos = atomicAdd(&taken, k);
+        if (pos + k <= kPaintList) {                     // those that fit fill the list without gaps
+          atomicMax(&listed, pos + k);
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            for (; w[q]; w[q] &= w[q] - 1) list[pos++] = at + 32u * q + (uint32_t)(__ffs(w[q]) - 1);
+        }
+      }
+      if (one_tab && !have_tab) ball_rows(tab, 0, side2, rr, r2max);
+      have_tab = true;
+      left = __syncthreads_or((w[0] | w[1] | w[2] | w[3]) != 0u);
+      const int count = listed;
+      for (int e0 = 0; e0 < side2; e0 += kRows) {
+        const int ne = min(kRows, side2 - e0);
+        if (!one_tab) {
+          ball_rows(tab, e0, ne, rr, r2max);
+          __syncthreads();
+        }
+        const int step_c = blockDim.x / ne, step_e = blockDim.x % ne;
+        int c = (int)threadIdx.x / ne, e = (int)threadIdx.x % ne;
+        while (c < count) {
+          const uint32_t v = tab[e], p = list[c];
+          if (v != 0xffffffffu) {
+            int z = (int)(p >> 20) + (int)(v >> 21) - 1023, y = (int)((p >> 10) & 1023u) + (int)((v >> 10) & 2047u) - 1023;
+            bool in = true;
+            if (periodic) {
+              z += z < 0 ? n : (z >= n ? -n : 0);
+              y += y < 0 ? n : (y >= n ? -n : 0);
+            } else {
+              in = z >= 0 && z < n && y >= 0 && y < n;
+            }
+            if (in) es::paint_row(z, y, (int)(p & 1023u), (int)(v & 1023u), n, periodic, flags);
+          }
+          c += step_c;
+          e += step_e;
+          if (e >= ne) { e -= ne; ++c; }
+        }
+        __syncthreads();
+      }
+      if (threadIdx.x == 0) taken = listed = 0;
+      __syncthreads();
+    }
+  }
+}
+
 __global__ void __launch_bounds__(256) paint_kernel(const uint32_t* __restrict__ centres, const unsigned* count,
                                                     uint32_t* flags, int n, int r2max, int periodic) {
   __shared__ uint32_t tab[kPaintTab];
@@ -283,45 +380,19 @@ __global__ void __launch_bounds__(256) paint_kernel(const uint32_t* __restrict__
   const uint32_t last_mask = last_bits == 32 ? 0xffffffffu : (1u << last_bits) - 1u;
   const uint32_t words = (uint32_t)n * n * nw;          // at most 1024^2 * 32
   const int lane = threadIdx.x & 31;
-  if ((long)cnt * kPaintSparse < (long)n * n * n) {
-    // words dealt to the warps in turn (four neighbours at a time in large boxes, whose words outnumber
-    // the warps), so that a cluster of centres is shared by many warps
-    const uint32_t nwarps = gridDim.x * (blockDim.x / 32);
-    const uint32_t warp = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
-    const int sh = words > 32u * nwarps ? 2 : 0;
-    for (uint32_t g = warp; (g << sh) < words; g += (32u >> sh) * nwarps) {
-      const uint32_t i = ((g + (uint32_t)(lane >> sh) * nwarps) << sh) + (uint32_t)(lane & ((1 << sh) - 1));
-      uint32_t w = 0u, v0 = 0u;
-      if (i < words) {
-        const uint32_t row = i / (uint32_t)nw, t = i % (uint32_t)nw;
-        w = centres[i] & ((int)t == nw - 1 ? last_mask : 0xffffffffu);
-        v0 = row * (uint32_t)n + 32u * t;
-      }
-      unsigned have = __ballot_sync(0xffffffffu, w != 0u);
-      while (have) {
-        const int src = __ffs(have) - 1;
-        have &= have - 1;
-        const uint32_t vs = __shfl_sync(0xffffffffu, v0, src);
-        for (uint32_t ws = __shfl_sync(0xffffffffu, w, src); ws; ws &= ws - 1)
-          es::paint_ball(vs + (uint32_t)(__ffs(ws) - 1), n, r2max, periodic, flags);
-      }
-    }
-    return;
-  }
   int rr = es::isqrt_dev(r2max);
   const int reach = periodic ? n / 2 : n - 1;           // farther offsets only repeat or leave the box
   if (rr > reach) rr = reach;
+  if ((long)cnt * kPaintSparse < (long)n * n * n) {
+    paint_centres(tab, rr, r2max, centres, flags, n, nw, last_mask, periodic);
+    return;
+  }
   const int side = 2 * rr + 1, slot = lane & 7;
   const uint32_t groups = gridDim.x * (blockDim.x / 8);
   for (int e0 = 0; e0 < side * side; e0 += kPaintTab) {
     const int ne = min(kPaintTab, side * side - e0);
     __syncthreads();
-    for (int e = threadIdx.x; e < ne; e += blockDim.x) {
-      const int dz = (e0 + e) / side - rr, dy = (e0 + e) % side - rr;
-      const int rem = r2max - dz * dz - dy * dy;
-      tab[e] = rem < 0 ? 0xffffffffu
-                       : ((uint32_t)(dz + 1023) << 21) | ((uint32_t)(dy + 1023) << 10) | (uint32_t)min(es::isqrt_dev(rem), 1023);
-    }
+    ball_rows(tab, e0, ne, rr, r2max);
     __syncthreads();
     for (uint32_t g0 = blockIdx.x * (blockDim.x / 8); g0 < words; g0 += groups) {     // uniform over the CTA
       const uint32_t g = g0 + (threadIdx.x >> 3);

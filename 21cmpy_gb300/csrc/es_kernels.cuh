@@ -345,6 +345,21 @@ template <int N> __device__ __forceinline__ void put_centres(uint16_t* bits, siz
   bits[row * (2 * ((N + 31) / 32)) + pair / 8] = (uint16_t)(spread16(even & 0xFFu) | (spread16(odd & 0xFFu) << 1));
 }
 
+// Voxels cx - w .. cx + w of row (z, y) in the pair-major bitmap; periodic wraps, otherwise clips to the row.
+__device__ __forceinline__ void paint_row(int z, int y, int cx, int w, int n, int periodic, uint32_t* flags) {
+  const long rb = ((long)z * n + y) * n;
+  int x0 = cx - w, x1 = cx + w;
+  if (periodic) {
+    if (x1 - x0 + 1 >= n) { set_bits(flags, rb, rb + n - 1); return; }
+    if (x0 < 0) { set_bits(flags, rb + x0 + n, rb + n - 1); x0 = 0; }
+    if (x1 >= n) { set_bits(flags, rb, rb + x1 - n); x1 = n - 1; }
+  } else {
+    if (x0 < 0) x0 = 0;
+    if (x1 > n - 1) x1 = n - 1;
+  }
+  set_bits(flags, rb + x0, rb + x1);
+}
+
 // Sphere painting (update_sphere_kernel, find_bubbles.cu:73-102), one warp per centre: every cell
 // within integer |d|^2 <= r2max of voxel v (linear index, x fastest) is set in the pair-major
 // bitmap; lanes split the (dz, dy) rows of the ball; periodic wraps, otherwise clips to the box.
@@ -360,17 +375,7 @@ __device__ __forceinline__ void paint_ball(uint32_t v, int n, int r2max, int per
     int z = cz + dz, y = cy + dy;
     if (periodic) { z = ((z % n) + n) % n; y = ((y % n) + n) % n; }
     else if (z < 0 || z >= n || y < 0 || y >= n) continue;
-    const long rb = ((long)z * n + y) * n;
-    int x0 = cx - w, x1 = cx + w;
-    if (periodic) {
-      if (x1 - x0 + 1 >= n) { set_bits(flags, rb, rb + n - 1); continue; }
-      if (x0 < 0) { set_bits(flags, rb + x0 + n, rb + n - 1); x0 = 0; }
-      if (x1 >= n) { set_bits(flags, rb, rb + x1 - n); x1 = n - 1; }
-    } else {
-      if (x0 < 0) x0 = 0;
-      if (x1 > n - 1) x1 = n - 1;
-    }
-    set_bits(flags, rb + x0, rb + x1);
+    paint_row(z, y, cx, w, n, periodic, flags);
   }
 }
 
