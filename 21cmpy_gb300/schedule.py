@@ -159,9 +159,13 @@ def pk_k2_thresholds(n: int, box_len: float, edges: np.ndarray) -> np.ndarray:
     dk = float(delta_k(box_len))
     kmax2 = 3 * (n // 2) ** 2
     e = np.asarray(edges, dtype=np.float64)
-    if not np.isfinite(e).all():
-        raise ValueError("bin edges must be finite")
-    m = np.minimum(np.floor((e / dk) ** 2), kmax2 + 8.0).astype(np.int64) + 2
+    with np.errstate(over="ignore"):
+        q = (e / dk) ** 2
+    if np.isnan(q).any():
+        raise ValueError("bin edges must be numbers")
+    if np.isinf(q).any():
+        raise OverflowError("bin edges must be finite, their squares in units of dk included")
+    m = np.minimum(np.floor(q), kmax2 + 8.0).astype(np.int64) + 2
     m[e < 0] = -1
     while True:                                     # at most a few steps: down to the last m with dk sqrt(m) <= edge
         over = (m >= 0) & (dk * np.sqrt(np.maximum(m, 0)) > e)
