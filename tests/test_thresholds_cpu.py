@@ -1,5 +1,6 @@
 """P(k) thresholds: the integers of the definition, edge by edge, and the edges that are refused."""
 import math
+import timeit
 
 import numpy as np
 import pytest
@@ -20,7 +21,7 @@ def test_edges_without_a_square_are_refused(bad, error, count):
 
 
 @pytest.mark.parametrize("n", [16, 128, 1024])
-@pytest.mark.parametrize("count", [1, 2, 15, 31, 32, 33, 64, 128])
+@pytest.mark.parametrize("count", [1, 2, 15, 55, 56, 57, 128])
 def test_thresholds_are_those_of_the_definition(n, count):
     rng = np.random.default_rng(n + count)
     L = 1.37 * n
@@ -38,3 +39,11 @@ def test_thresholds_are_those_of_the_definition(n, count):
 
 def test_no_edges():
     assert sch.pk_k2_thresholds(32, 50.0, np.zeros(0)).shape == (0,)
+
+
+def test_one_edge_costs_less_than_a_hundred():
+    def time(count):
+        edges = sch.pk_edges(64, 96.0, count)
+        return min(timeit.repeat(lambda: sch.pk_k2_thresholds(64, 96.0, edges), number=100, repeat=5))
+
+    assert time(1) < 0.5 * time(100)
