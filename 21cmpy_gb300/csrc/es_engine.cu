@@ -717,6 +717,16 @@ int reuse_staging(es_plan* p) {
   return ES_OK;
 }
 
+// whether [q, q + bytes) touches one of a plan's spectra
+bool in_spectra(const es_plan* p, const void* q, size_t bytes) {
+  const size_t N = p->n;
+  const uintptr_t a = (uintptr_t)q, b = a + bytes;
+  auto meets = [&](const float2* s, size_t n) { return a < (uintptr_t)(s + n) && (uintptr_t)s < b; };
+  for (int i = 0; i < p->nspec; ++i)
+    if (meets(p->spec[i], N * N * (N / 2)) || meets(p->spec_nyq[i], N * N)) return true;
+  return false;
+}
+
 // the spectrum that the plain transforms use (the first one of a plan for transforms alone)
 int fft_spec(const es_plan* p) { return p->fft_only ? 0 : SPEC_T; }
 
@@ -1251,6 +1261,16 @@ int ic_sampled_fields(es_plan* big, const void* half, es_plan* small, int filter
     return fail(ES_E_ARG, "ic_sampled_fields: bad arguments");
   for (int i = 0; i < count; ++i)
     if (!out[i]) return fail(ES_E_ARG, "ic_sampled_fields: NULL output");
+  // the fold reads mirror rows while other CTAs write small's spectra, and the inverses read those one after another
+  if (big == small) return fail(ES_E_ARG, "ic_sampled_fields: big and small are the same plan");
+  const size_t N = big->n, h3 = (size_t)small->n * small->n * small->n;
+  if (half && in_spectra(small, half, N * N * (N / 2 + 1) * sizeof(float2)))
+    return fail(ES_E_ARG, "ic_sampled_fields: half lies in small's workspace");
+  if (!half && in_spectra(small, big->spec[fft_spec(big)], N * N * (N / 2) * sizeof(float2)))
+    return fail(ES_E_ARG, "ic_sampled_fields: big and small share a workspace");
+  for (int i = 0; i < count; ++i)
+    if (in_spectra(small, out[i], h3 * sizeof(float)))
+      return fail(ES_E_ARG, "ic_sampled_fields: an output lies in small's workspace");
   DeviceGuard g(big->device);
   cudaStream_t s = (cudaStream_t)stream;
   const int f = fft_spec(big);

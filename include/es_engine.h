@@ -163,7 +163,8 @@ int es_fft_c2r(es_plan* plan, const void* in_half, float* out, void* stream);
 int es_fft_c2r_scaled(es_plan* plan, const void* in_half, float scale, float* out, void* stream);
 
 /* A plan for transforms alone, on a workspace the caller owns (device memory, 256-byte aligned,
- * es_fft_plan_bytes(n, spectra) bytes; it must outlive the plan) with `spectra` (1..4) spectra in it,
+ * es_fft_plan_bytes(n, spectra) bytes; it must outlive the plan, and no input or output of a call may
+ * lie in it) with `spectra` (1..4) spectra in it,
  * and the table twiddles[m] = exp(-2 pi i m / n), m < n (device complex64).  Creating it launches one
  * memset on the stream and allocates nothing on the device.  It serves es_fft_r2c, es_fft_c2r(_scaled),
  * es_fft_forward, es_density, ic_sampled_fields, the options, es_plan_check and es_plan_destroy; es_forward,
@@ -334,7 +335,8 @@ int ic_shape(int n, float box_len, const void* in_half, int component, int filte
  * every p-th cell is folding the spectrum p-fold onto itself, so the shaped spectrum is folded to
  * HII_DIM^3 in one reading and only HII_DIM^3 inverse transforms follow.  big: a plan of DIM (its
  * own spectrum, es_fft_forward, is used when half is NULL); small: an es_fft_plan of HII_DIM with at
- * least count spectra; DIM must be a multiple of HII_DIM.  out[i]: device float HII_DIM^3, times scale. */
+ * least count spectra; DIM must be a multiple of HII_DIM.  out[i]: device float HII_DIM^3, times scale.
+ * ES_E_ARG if big and small are one plan, or if half, an out[i] or big's spectrum lies in small's workspace. */
 int ic_sampled_fields(es_plan* big, const void* half, es_plan* small, int filter_type, float R, int ref_compat, int first,
                       int count, float scale, float* const* out, void* stream);
 int ic_subsample(int dim, int hii_dim, float pixel_factor, float scale, const float* large, float* small,
