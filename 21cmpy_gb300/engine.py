@@ -319,10 +319,13 @@ def sampled_fields(big: ExcursionSetPlan, half, small: FftPlan, first: int, coun
         if half.dtype != torch.complex64 or tuple(half.shape) != (n, n, n // 2 + 1) or half.device != big.device \
                 or not half.is_contiguous():
             raise ValueError("half must be a contiguous complex64 (n, n, n/2+1) device tensor")
+    stream = torch.cuda.current_stream(small.device)
+    if half is None and isinstance(big, FftPlan):
+        big._on(stream)                  # its workspace is read here too
     outs = [torch.empty((small.n,) * 3, dtype=torch.float32, device=small.device) for _ in range(count)]
     ptrs = (C.c_void_p * count)(*[o.data_ptr() for o in outs])
     rc = small.lib.ic_sampled_fields(big.handle, None if half is None else _ptr(half), small.handle, int(filter_type),
                                      C.c_float(float(R)), int(ref_compat), int(first), int(count),
-                                     C.c_float(float(np.float32(scale))), ptrs, small._on(None))
+                                     C.c_float(float(np.float32(scale))), ptrs, small._on(stream))
     _lib.check("ic_sampled_fields", rc, small.lib)
     return outs
