@@ -261,7 +261,10 @@ class FftPlan(ExcursionSetPlan):
         handle = C.c_void_p()
         with torch.cuda.device(self.device):
             if nbytes:
-                self._ws = torch.empty(nbytes, dtype=torch.uint8, device=self.device)
+                try:
+                    self._ws = torch.empty(nbytes, dtype=torch.uint8, device=self.device)
+                except torch.OutOfMemoryError as e:
+                    raise _lib.EngineError("es_fft_plan_create", _lib.ES_E_NOMEM, str(e)) from e
                 self._tw = _twiddles(self.n, self.device)
             rc = self.lib.es_fft_plan_create(self.n, self.box_len, self.spectra, _ptr(self._tw) if nbytes else None,
                                              _ptr(self._ws) if nbytes else None, nbytes,
