@@ -64,9 +64,9 @@ class InitialConditions:
 
     @property
     def plan(self):
-        """A full plan of DIM^3 boxes, made at first use (the boxes here need transforms alone)."""
+        """A full plan of DIM^3 boxes, made at first use (the boxes here need transforms alone); None once closed."""
         from .engine import ExcursionSetPlan
-        if self._plan is None:
+        if self._plan is None and self._fft is not None:
             self._plan = ExcursionSetPlan(self.dim, self.box_len, max_radii=1, device=self.device)
         return self._plan
 
