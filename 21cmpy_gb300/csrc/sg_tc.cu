@@ -80,7 +80,7 @@ template <int CIN, int COUT> struct Layout {
   static constexpr int W_OFF = (RING_BYTES + 127) / 128 * 128;
   static constexpr int BAR_OFF = W_OFF + W_BYTES;
   static constexpr int NBARS = 2 * YS + 2 * S + 1;    // full[YS], sfree[YS], done[S], tfree[S], drain
-  static constexpr int BYTES = BAR_OFF + NBARS * 8 + 16 + 1024;   // + tmem slot, abort, alignment
+  static constexpr int BYTES = BAR_OFF + NBARS * 8 + 16 + 1024;   // + tmem slot, abort, groups issued, alignment
   static_assert(VOX == 64 || VOX == 32, "a voxel is one swizzle span");
   static_assert(W_BYTES % 16 == 0, "16-byte aligned regions");
   static_assert(3 * COUT <= 256 && COUT % 16 == 0, "N = 3 COUT must be a valid M = 128 MMA width");
@@ -337,12 +337,7 @@ __global__ void __launch_bounds__(CONV_THREADS, 1) conv_tc_kernel(const __grid_c
     if (lane == 0) {
       for (; !walk.done(); issue_group())
         if (issued >= YS && !bar_wait(&sfree[issued % YS], (uint32_t)((issued / YS - 1) & 1), abort)) break;
-      // no copy outlives the CTA: after an abort every group issued lands first (bounded; otherwise the MMA
-      // warp has seen them all)
-      if (*abort)
-        for (int q = issued > YS ? issued - YS : 0; q < issued; ++q)
-          for (long i = 0; i < kSpin && !bar_try(&full[q % YS], (uint32_t)((q / YS) & 1)); ++i) {
-          }
+      abort[1] = issued;
     }
   } else if (warp == CONV_MMA_WARP) {
     {
@@ -501,6 +496,15 @@ __global__ void __launch_bounds__(CONV_THREADS, 1) conv_tc_kernel(const __grid_c
 
   tc_before();
   __syncthreads();
+  // No copy outlives the CTA: the MMA warp has seen every group land, or a role has aborted, which is known only
+  // here (the producer may have left its loop before) and then they land first (bounded).  The number issued comes
+  // through shared memory: kept in a register to here it changed the whole kernel's schedule (128^3 forward 953 -> 960 us)
+  if (threadIdx.x == 0 && *abort) {
+    const int groups = abort[1];
+    for (int q = groups > YS ? groups - YS : 0; q < groups; ++q)
+      for (long i = 0; i < kSpin && !bar_try(&full[q % YS], (uint32_t)((q / YS) & 1)); ++i) {
+      }
+  }
   if (warp == 0) {
     __syncwarp();
     tc_after();
@@ -548,7 +552,7 @@ template <int CIN, int COUT> struct WLayout {
   static constexpr int A_END = XRING + (CIN == 16 ? XGROUP : 0);
   static constexpr int BAR_OFF = ((D_END > A_END ? D_END : A_END) + 15) / 16 * 16;
   static constexpr int NBARS = 2 * wg::XS + 2 * wg::DSL + 1;    // xfull, xfree, dfull, dfree, done
-  static constexpr int BYTES = BAR_OFF + NBARS * 8 + 16 + 1024;
+  static constexpr int BYTES = BAR_OFF + NBARS * 8 + 16 + 1024;   // + tmem slot, abort, items issued, alignment
   static_assert(NCOLS % 16 == 0 && NCOLS <= 256, "N = 3 COUT must be a valid M = 128 MMA width");
   static_assert(XGROUP % 512 == 0 && DROW % 512 == 0, "rows start on a whole swizzle pattern");
   static_assert(BYTES <= 232448, "shared memory per CTA");
@@ -678,15 +682,8 @@ __global__ void __launch_bounds__(wg::WG_THREADS, 1) wgrad_tc_kernel(const __gri
         for (int y = yb; y < ye && ok; ++y) ok = issue_x(z, (y + 1) % N) && issue_d(z * N + y);
         r = z * N + ye;
       }
-      // after an abort, what is under way lands before the CTA leaves (bounded)
-      if (*abort) {
-        for (int q = nx > wg::XS ? nx - wg::XS : 0; q < nx; ++q)
-          for (long i = 0; i < kWSpin && !bar_try(&xfull[q % wg::XS], (uint32_t)((q / wg::XS) & 1)); ++i) {
-          }
-        for (int q = nd > wg::DSL ? nd - wg::DSL : 0; q < nd; ++q)
-          for (long i = 0; i < kWSpin && !bar_try(&dfull[q % wg::DSL], (uint32_t)((q / wg::DSL) & 1)); ++i) {
-          }
-      }
+      abort[1] = nx;
+      abort[2] = nd;
     }
   } else if (warp == CONV_MMA_WARP) {
     // ---------------------------------------------------------------- MMA issue
@@ -767,6 +764,16 @@ __global__ void __launch_bounds__(wg::WG_THREADS, 1) wgrad_tc_kernel(const __gri
 
   tc_before();
   __syncthreads();
+  // no copy outlives the CTA (as in the convolutions)
+  if (threadIdx.x == 0 && *abort) {
+    const int nx = abort[1], nd = abort[2];
+    for (int q = nx > wg::XS ? nx - wg::XS : 0; q < nx; ++q)
+      for (long i = 0; i < kWSpin && !bar_try(&xfull[q % wg::XS], (uint32_t)((q / wg::XS) & 1)); ++i) {
+      }
+    for (int q = nd > wg::DSL ? nd - wg::DSL : 0; q < nd; ++q)
+      for (long i = 0; i < kWSpin && !bar_try(&dfull[q % wg::DSL], (uint32_t)((q / wg::DSL) & 1)); ++i) {
+      }
+  }
   if (warp == 0) {
     __syncwarp();
     tc_after();
