@@ -33,14 +33,26 @@ namespace ic {
 __device__ __forceinline__ int wrapk(int m, int n) { return m > n / 2 ? m - n : m; }
 
 // first index i in [1, tn) with K[i] >= k (K[0] < k holds for every k > 0 of the box; tn - 1 if there is
-// none), from where a log-spaced table would have it: the search steps from there until it is
-// right, whatever the spacing
+// none): right there or one beside where a log-spaced table would have it, or else by halving what is left on that
+// side.  512^3 with 4096 entries: log-spaced 233 us, linear 350 (one step after the other from the guess: 16.3 ms).
 __device__ __forceinline__ int upper(const float* K, int tn, float k, float l0, float per) {
   const float g = (__log2f(k) - l0) * per + 1.0f;
-  int i = g >= 1.0f && g < (float)(tn - 1) ? (int)g : (g >= 1.0f ? tn - 1 : 1);
-  while (i < tn - 1 && K[i] < k) ++i;
-  while (i > 1 && K[i - 1] >= k) --i;
-  return i;
+  const int i = g >= 1.0f && g < (float)(tn - 1) ? (int)g : (g >= 1.0f ? tn - 1 : 1);
+  int lo, hi;                                           // the index lies in (lo, hi]
+  if (K[i] < k) {
+    lo = i;
+    hi = min(i + 1, tn - 1);
+    if (K[hi] < k) { lo = hi; hi = tn - 1; }
+  } else {
+    hi = i;
+    lo = i - 1;
+    if (K[lo] >= k) { hi = max(lo, 1); lo = 0; }
+  }
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (K[mid] >= k) hi = mid; else lo = mid;
+  }
+  return hi;
 }
 
 // The rows (+-k0, +-k1) of a quad: P depends on |k| alone, so what one element needs (two square roots,
