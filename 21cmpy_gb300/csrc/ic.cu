@@ -220,9 +220,9 @@ __global__ void __launch_bounds__(544, 2) fold_kernel(int n, int h, float dk, co
 #pragma unroll
           for (int c = 0; c < NC; ++c) {
             const int comp = first + c;
-            if (comp < 0) {
-              acc[s][c].x += x;
-              acc[s][c].y += y;
+            if (comp < 0) {                             // the product unrounded: x is rounded for the other components
+              acc[s][c].x = fmaf(v[s].x, W, acc[s][c].x);
+              acc[s][c].y = fmaf(up ? -v[s].y : v[s].y, W, acc[s][c].y);
             } else {
               const float f = comp == 0 ? (s & 1 ? -f0 : f0) : comp == 1 ? (s & 2 ? -f1 : f1) : f2;
               acc[s][c].x -= f * y;
