@@ -476,11 +476,25 @@ __device__ __forceinline__ void pk_bin_columns(const float2* g, int ck2, unsigne
   pk_bin_segment<N, KS>([&](int k) { return g[k * TI + col]; }, seg, ck2, wgt, thr, nbins, dk, volume, sum_p, sum_k, count);
 }
 
+// A float32 sum and what its additions have rounded away (two-sum: s + e is exact after each).
+struct ExactSum {
+  float s = 0.f, e = 0.f;
+  __device__ __forceinline__ void add(float x) {
+    const float t = __fadd_rn(s, x), b = __fsub_rn(t, s);
+    e = __fadd_rn(e, __fadd_rn(__fsub_rn(s, __fsub_rn(t, b)), __fsub_rn(x, b)));
+    s = t;
+  }
+  __device__ __forceinline__ float value() const { return s + e; }
+};
+
 // Per-CTA bins (fixed warp order) -> partials -> the last CTA of each group of consecutive CTAs adds
 // the group's partials -> the last group adds the groups', each in a fixed order, and writes ps_ave,
 // k_ave and the count (rounded to float32 once, at the end).  About sqrt(grid) CTAs form a group, so
 // either step reads ~20 partials per value, all in flight at once: the single last CTA that read all
 // 304 of them one after the other took 45 us of the 256^3 pass with 20 bins and 160 us with 100.
+// The steps carry their rounding along (ExactSum): by plain float32 additions, one after the other, they were
+// the larger part of a bin's error (relative rms at 128^3 with 20 bins 9.6e-8, now 8.3e-8; 8.5e-8 by the
+// butterfly of that last CTA's lanes).  Float64 does the same for 4 us more at 256^3 with 100 bins.
 constexpr int kPkGroups = 48;                         // arrival counters of the groups, from counter[16]
 template <int T, int NWB = T / 32>                    // NWB: warps that have bins
 __device__ __forceinline__ void pk_finish(float* bins, const OpArgs& a) {
@@ -493,9 +507,9 @@ __device__ __forceinline__ void pk_finish(float* bins, const OpArgs& a) {
   for (int idx = threadIdx.x; idx < nb3; idx += T) {
     const int q = idx / a.nbins, bin = idx % a.nbins;
     if (q < 2) {
-      float s = 0.f;
-      for (int w = 0; w < NWB; ++w) s += bins[w * PK_MAX_BINS * 3 + q * PK_MAX_BINS + bin];
-      a.partials[(size_t)blockIdx.x * nb3 + idx] = s;
+      ExactSum s;
+      for (int w = 0; w < NWB; ++w) s.add(bins[w * PK_MAX_BINS * 3 + q * PK_MAX_BINS + bin]);
+      a.partials[(size_t)blockIdx.x * nb3 + idx] = s.value();
     } else {
       unsigned s = 0u;
       for (int w = 0; w < NWB; ++w) s += pk_counts(bins + w * PK_MAX_BINS * 3)[bin];
@@ -506,10 +520,10 @@ __device__ __forceinline__ void pk_finish(float* bins, const OpArgs& a) {
   // `parts` partials starting at src: value idx, as float or (counts) exact unsigned
   auto add_up = [&](const float* src, int parts, int idx) {
     if (idx < 2 * a.nbins) {
-      float s = 0.f;
+      ExactSum s;
 #pragma unroll 8
-      for (int c = 0; c < parts; ++c) s += __ldcg(src + (size_t)c * nb3 + idx);
-      return s;
+      for (int c = 0; c < parts; ++c) s.add(__ldcg(src + (size_t)c * nb3 + idx));
+      return s.value();
     }
     unsigned s = 0u;                                  // at most 1024^3 modes
 #pragma unroll 8
