@@ -156,7 +156,7 @@ Layout layout(int n, int max_radii, size_t partial_floats) {
   L.dR0 = take(N * N * N * 4);
   L.dR1 = take(N * N * N * 4);
   L.flags = take(N * N * N / 8);
-  L.centres = take(N * N * N * 4);
+  L.centres = take(N * N * N * 4);      // the bitmap takes N^3 / 8 of it; the sizes stated for plans count a word a cell
   L.wtab = take((size_t)max_radii * k2n * 4);
   L.partials = take(partial_floats * 4);
   L.counters = take(256);
@@ -642,7 +642,8 @@ void set_maps(es::OpArgs& a, const es_plan* p, int in, int out, bool z, bool col
 // a pass lasts 4-40 us, of which launch and set-up are a good part.  At 512^3 it lasts 200-260 us and is
 // bound by DRAM, which likes all CTAs to walk the spectrum in step: CTAs that start as the previous
 // kernel's leave lose more by that than the launch gaps cost (whole box 28.8 ms without, 31.2 with).  The
-// synchronous passes have no pdl_wait.
+// figures are of one plan on the GPU: three at 256^3 side by side lose 6 % by it (52 boxes 146.1 ms, 137.2 without),
+// three at 64^3 or 128^3 gain (205 / 281 and 389 / 404 us a box).  The synchronous passes have no pdl_wait.
 bool uses_pdl(const es_plan* p) { return p->col_variant == 1 && p->n <= 256; }
 
 template <class... P, class... A>

@@ -232,7 +232,7 @@ __device__ __forceinline__ f32x2 erfc_sum_pair(f32x2 xv) {
   const float2 x = upk2(xv);
   const float z0 = fabsf(x.x), z1 = fabsf(x.y);
   const float2 d = upk2(fma2(pk2(z0, z1), bc2(0.5f), bc2(1.0f)));
-  const f32x2 T = pk2(rcp_approx(d.x), rcp_approx(d.y));   // divisors in [1, 11]: normal numbers
+  const f32x2 T = pk2(rcp_approx(d.x), rcp_approx(d.y));   // divisors of at least 1; below 2^126 their reciprocals are normal numbers
   f32x2 P = bc2(0.17087277f * L2E);
   P = fma2(P, T, bc2(-0.82215223f * L2E));
   P = fma2(P, T, bc2(1.48851587f * L2E));
