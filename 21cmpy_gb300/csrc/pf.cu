@@ -133,8 +133,9 @@ __global__ void __launch_bounds__(256) move_mass_kernel(int dim, int sw, const f
 // and at most 2^-17, and remainder * 2^32 + 1.5 * 2^23 rounds it to an integer the same way, ties to even;
 // hi * 2^16 + lo is then __float2ll_rn(m * 2^32), since the first part is even.  Both parts are summed as 32-bit
 // integers (P^3 masses of at most 2^22: below 2^31 for P = 4, and |m| < 16 is asked for with P = 8).
-// Larger masses, NaN, and targets that are neither A nor B (displacements beyond float32's resolution
-// of a cell) take the cell-by-cell way for that thread.
+// With a larger mass or NaN a thread adds up once more by 64-bit conversions (wide_sums; where every thread does, 512^3 ->
+// 64^3 takes 391 us, 957 by an atomic per cell and 449 by runs of 8 cells); targets that are neither A nor B
+// (displacements beyond float32's resolution of a cell) go cell by cell.
 //
 // 512^3 -> 128^3: 493 us a run of 8 cells per lane with ~4 atomics each, 147 us this way (0.57 GB: 84 us).
 template <int P> struct Row { float v[P]; };
@@ -151,6 +152,38 @@ template <int P> __device__ __forceinline__ Row<P> load_row(const float* p) {
     }
   }
   return r;
+}
+
+// The sums q [axis 0][axis 1][axis 2] (0: total, 1: A's share) with a 64-bit conversion per mass, whatever its
+// size: modulo 2^64, as the atomics add them.
+template <int P>
+__device__ __forceinline__ void wide_sums(const float* cell, int dim, int planes, float g0, unsigned b0, unsigned b1, unsigned b2,
+                                       unsigned long long (&q)[2][2][2]) {
+#pragma unroll
+  for (int i = 0; i < 8; ++i) q[i >> 2][(i >> 1) & 1][i & 1] = 0ull;
+#pragma unroll 1
+  for (int k0 = 0; k0 < planes; ++k0) {
+    const bool in0 = !((b0 >> k0) & 1u);
+#pragma unroll 1
+    for (int k1 = 0; k1 < P; ++k1) {
+      const bool in1 = !((b1 >> k1) & 1u);
+      const Row<P> r = load_row<P>(cell + ((size_t)k0 * dim + k1) * dim);
+      unsigned long long t[2] = {0ull, 0ull};
+#pragma unroll
+      for (int k = 0; k < P; ++k) {
+        const unsigned long long v = (unsigned long long)__float2ll_rn(__fadd_rn(1.0f, __fmul_rn(g0, r.v[k])) * kFix);
+        t[0] += v;
+        t[1] += (b2 >> k) & 1u ? 0ull : v;
+      }
+#pragma unroll
+      for (int z = 0; z < 2; ++z) {
+        q[0][0][z] += t[z];
+        q[0][1][z] += in1 ? t[z] : 0ull;
+        q[1][0][z] += in0 ? t[z] : 0ull;
+        q[1][1][z] += in0 && in1 ? t[z] : 0ull;
+      }
+    }
+  }
 }
 
 template <int P>
@@ -185,46 +218,6 @@ __global__ void __launch_bounds__(256) move_cells_kernel(int sw, int parts, cons
   axis(pos + h1 * P, vyv, P, t1a, t1b, b1);
   axis(pos + h2 * P, vzv, P, t2a, t2b, b2);
   const float* cell = delta + ((size_t)(h0 * P + k0a) * dim + h1 * P) * dim + h2 * P;
-  // sums [axis 0][axis 1][axis 2], 0: total, 1: A's share; hi and lo parts
-  int hi[2][2][2] = {}, lo[2][2][2] = {};
-  if (ok) {
-    int m2[P];
-#pragma unroll
-    for (int k = 0; k < P; ++k) m2[k] = (b2 >> k) & 1u ? 0 : -1;
-    for (int k0 = 0; k0 < planes; ++k0) {
-      int ph[2][2] = {}, pl[2][2] = {};
-#pragma unroll
-      for (int k1 = 0; k1 < P; ++k1) {
-        const Row<P> r = load_row<P>(cell + ((size_t)k0 * dim + k1) * dim);
-        int th = 0, tl = 0, ah = 0, al = 0;
-#pragma unroll
-        for (int k = 0; k < P; ++k) {
-          const float mass = __fadd_rn(1.0f, __fmul_rn(g0, r.v[k]));
-          ok = ok && fabsf(mass) < kLimit;                           // false for NaN, and then for good
-          const float up = __fadd_rn(mass, 192.0f);
-          const float low = __fsub_rn(mass, __fsub_rn(up, 192.0f));
-          const int qh = __float_as_int(up) - 0x43400000, ql = __float_as_int(fmaf(low, kFix, 12582912.0f)) - 0x4B400000;
-          th += qh;
-          tl += ql;
-          ah += qh & m2[k];
-          al += ql & m2[k];
-        }
-        const int m1 = (b1 >> k1) & 1u ? 0 : -1;
-        ph[0][0] += th; pl[0][0] += tl; ph[0][1] += ah; pl[0][1] += al;
-        ph[1][0] += th & m1; pl[1][0] += tl & m1; ph[1][1] += ah & m1; pl[1][1] += al & m1;
-      }
-      const int m0 = (b0 >> k0) & 1u ? 0 : -1;
-#pragma unroll
-      for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          hi[0][i][j] += ph[i][j];
-          lo[0][i][j] += pl[i][j];
-          hi[1][i][j] += ph[i][j] & m0;
-          lo[1][i][j] += pl[i][j] & m0;
-        }
-    }
-  }
   if (!ok) {
     for (int k0 = 0; k0 < planes; ++k0)
       for (int k1 = 0; k1 < P; ++k1)
@@ -237,12 +230,50 @@ __global__ void __launch_bounds__(256) move_cells_kernel(int sw, int parts, cons
         }
     return;
   }
-  long long q[2][2][2];
+  // sums [axis 0][axis 1][axis 2], 0: total, 1: A's share; hi and lo parts
+  int hi[2][2][2] = {}, lo[2][2][2] = {}, m2[P];
+#pragma unroll
+  for (int k = 0; k < P; ++k) m2[k] = (b2 >> k) & 1u ? 0 : -1;
+  for (int k0 = 0; k0 < planes; ++k0) {
+    int ph[2][2] = {}, pl[2][2] = {};
+#pragma unroll
+    for (int k1 = 0; k1 < P; ++k1) {
+      const Row<P> r = load_row<P>(cell + ((size_t)k0 * dim + k1) * dim);
+      int th = 0, tl = 0, ah = 0, al = 0;
+#pragma unroll
+      for (int k = 0; k < P; ++k) {
+        const float mass = __fadd_rn(1.0f, __fmul_rn(g0, r.v[k]));
+        ok = ok && fabsf(mass) < kLimit;                             // false for NaN, and then for good
+        const float up = __fadd_rn(mass, 192.0f);
+        const float low = __fsub_rn(mass, __fsub_rn(up, 192.0f));
+        const int qh = __float_as_int(up) - 0x43400000, ql = __float_as_int(fmaf(low, kFix, 12582912.0f)) - 0x4B400000;
+        th += qh;
+        tl += ql;
+        ah += qh & m2[k];
+        al += ql & m2[k];
+      }
+      const int m1 = (b1 >> k1) & 1u ? 0 : -1;
+      ph[0][0] += th; pl[0][0] += tl; ph[0][1] += ah; pl[0][1] += al;
+      ph[1][0] += th & m1; pl[1][0] += tl & m1; ph[1][1] += ah & m1; pl[1][1] += al & m1;
+    }
+    const int m0 = (b0 >> k0) & 1u ? 0 : -1;
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        hi[0][i][j] += ph[i][j];
+        lo[0][i][j] += pl[i][j];
+        hi[1][i][j] += ph[i][j] & m0;
+        lo[1][i][j] += pl[i][j] & m0;
+      }
+  }
+  unsigned long long q[2][2][2];
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     const int x = i >> 2, y = (i >> 1) & 1, z = i & 1;
-    q[x][y][z] = (long long)hi[x][y][z] * 65536 + lo[x][y][z];
+    q[x][y][z] = (unsigned long long)((long long)hi[x][y][z] * 65536 + lo[x][y][z]);
   }
+  if (!ok) wide_sums<P>(cell, dim, planes, g0, b0, b1, b2, q);
   // totals -> B's shares, axis by axis
 #pragma unroll
   for (int i = 0; i < 2; ++i)
@@ -261,7 +292,7 @@ __global__ void __launch_bounds__(256) move_cells_kernel(int sw, int parts, cons
     const int x = i >> 2, y = (i >> 1) & 1, z = i & 1;
     if ((x || b0) && (y || b1) && (z || b2))
       atomicAdd(acc + ((unsigned)(x ? t0a : t0b) * usw + (unsigned)(y ? t1a : t1b)) * usw + (unsigned)(z ? t2a : t2b),
-                (unsigned long long)q[x][y][z]);
+                q[x][y][z]);
   }
 }
 

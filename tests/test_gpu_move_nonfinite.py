@@ -34,3 +34,25 @@ def test_same_bits_as_cell_by_cell(dim, sw, first, second, place):
             d.copy_(torch.from_numpy(delta))
             out.append(plan.move_mass(d, *v, init_growth=0.1, disp_scale=0.01, mass_factor=float(P ** 3)))
     assert torch.equal(out[0].view(torch.int32), out[1].view(torch.int32))
+
+
+@pytest.mark.parametrize("dim,sw", [(256, 128), (256, 64), (512, 64)])
+def test_large_masses_are_no_slower_than_cell_by_cell(dim, sw):
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    g = torch.Generator(device="cuda").manual_seed(dim + sw)
+    buf = torch.randn(dim ** 3 + 1, device="cuda", generator=g)
+    v = [torch.randn((sw,) * 3, device="cuda", generator=g) * 0.5 for _ in range(3)]
+    ms = []
+    with module("perturb").PerturbPlan(dim, sw) as plan:
+        for offset in (0, 1):                            # whole HII cells, cell by cell
+            d = buf[offset:offset + dim ** 3].view(dim, dim, dim)
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            for q in range(14):
+                if q == 4:
+                    a.record()
+                plan.move_mass(d, *v, init_growth=1e3, disp_scale=1.0 / sw, mass_factor=1.0)
+            b.record()
+            torch.cuda.synchronize()
+            ms.append(a.elapsed_time(b))
+    assert ms[0] <= 1.1 * ms[1], ms
